@@ -88,11 +88,43 @@ struct GradSpecJob {
 };
 
 // Serial reductions over a signal, in the CPU's order, into
-// out[0] = sum x, out[1] = sum (-1)^k (x - mean), out[2] = sum x*x.
+// out[0] = sum x, out[1] = sum (-1)^k (x - mean), out[2] = sum x*x,
+// out[3] = the first k with x[k]*x[k] != 0 (exact form; len if none).
 struct SumJob {
     VSig sig;
     double *out;
 };
+
+// Energy of the lag-aligned degraded signal (reference src/realign.zig:91-110
+// then src/audio.zig:132-136), the lag read on the device: out[0] = energy,
+// out[1] = aligned length. deg_stats: the whole signal's SumJob sums (out[2]
+// its energy, out[3] the first index with a nonzero energy term), or null.
+struct AlignedEnergyJob {
+    VSig deg;
+    int64_t ref_len;
+    const int64_t *lag;
+    double *out;
+    const double *deg_stats;
+};
+
+// applyLag drops -lag leading samples, or prepends lag zeros (which add +0 to
+// the sum), and leaves lags of 0 or beyond half the reference alone.
+__host__ __device__ inline void aligned_range(const AlignedEnergyJob &job, int64_t &skip, int64_t &alen) {
+    const int64_t lag = *job.lag;
+    const int64_t half_ref = job.ref_len / 2;
+    const int64_t mag = lag < 0 ? -lag : lag;
+    const int64_t L = job.deg.len;
+    skip = 0;
+    alen = L;
+    if (lag != 0 && mag <= half_ref) {
+        if (lag < 0) {
+            skip = -lag < L ? -lag : L;
+            alen = L - skip;
+        } else {
+            alen = L + lag;
+        }
+    }
+}
 
 // One spectrogram pair to prepare for comparison (reference
 // src/spectrogram.zig:69-80): in-place on ref[nb*nfr], deg[nb*nfd].

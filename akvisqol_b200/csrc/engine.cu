@@ -427,7 +427,10 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
     const size_t np = nfr / std::max<size_t>(1, P) + 1;
     const size_t n_global = host::fft_size_for(std::max(rl, dl));
     const size_t n_slice = host::fft_size_for(2 * P * H + 2);
+    const size_t sums = 2 * serial_sum_scratch(2, (int64_t)std::max(rl, dl)) +
+                        serial_sum_scratch((int)(2 * np), (int64_t)(2 * P * H + 2));
     size_t b = 8 * (rl + dl)                                   // inputs
+               + sums                                          // the exact form's serial sums
                + 16 * n_global + 16 * 1024                     // lag search and argmax parts
                + 8 * al                                        // aligned, scaled degraded signal
                + 8 * NB * (2 * nfr + 2 * nfd + 4 * width)      // spectrograms, prepared copies, plane
@@ -673,11 +676,19 @@ void Engine::prepare(size_t n, const double *const *refs, const size_t *ref_lens
 
 void Engine::launch_sums(const std::vector<SumJob> &sums) {
     if (sums.empty()) return;
-    const SumJob *d = upload(sums);
-    if (opt_.form != kFormExact)
-        launch_envelope_stats_tree(d, (int)sums.size(), arena_.alloc_n<double>(sums.size() * kTreeParts * 3), stream_);
-    else
-        launch_envelope_stats(d, (int)sums.size(), stream_);
+    if (opt_.form == kFormExact) {
+        launch_serial_sums(sums);
+        return;
+    }
+    launch_envelope_stats_tree(upload(sums), (int)sums.size(), arena_.alloc_n<double>(sums.size() * kTreeParts * 3),
+                               stream_);
+}
+
+void Engine::launch_serial_sums(const std::vector<SumJob> &sums) {
+    int64_t max_len = 0;
+    for (const SumJob &j : sums) max_len = std::max(max_len, j.sig.len);
+    launch_envelope_stats(upload(sums), (int)sums.size(), max_len,
+                          arena_.alloc(serial_sum_scratch((int)sums.size(), max_len)), stream_);
 }
 
 void Engine::lags(size_t njobs, const VSig *a, const VSig *b, bool raw, int64_t *h_lags, int32_t *status_out,
@@ -707,7 +718,7 @@ void Engine::lags(size_t njobs, const VSig *a, const VSig *b, bool raw, int64_t 
     std::vector<size_t> where;
     for (size_t i = 0; i < njobs; ++i)
         if (jobs[i].biggest > 0) run.push_back(jobs[i]), where.push_back(i);
-    if (!raw && !sums.empty()) launch_envelope_stats(upload(sums), (int)sums.size(), stream_);
+    if (!raw && !sums.empty()) launch_serial_sums(sums);
     int32_t *d_status = launch_lag_jobs(run, raw);
     int64_t *h = pinned_.alloc_n<int64_t>(njobs);
     int32_t *h_status = d_status ? pinned_.alloc_n<int32_t>(run.size()) : nullptr;
@@ -934,22 +945,21 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     int32_t *d_lstat = nullptr;    // FP32 form: per lag job, 1 when the f32 search left it undecided
     // aligned energies (read the lags on the device) of the listed pairs
     auto launch_aligned = [&](const std::vector<size_t> &pairs) {
-        std::vector<char> args;
-        const size_t asz = aligned_energy_args_size();
-        int na = 0;
+        std::vector<AlignedEnergyJob> jobs;
+        int64_t max_len = 0;
         for (size_t i : pairs) {
             PairState &s = ps[i];
             if (!s.live) continue;
-            args.resize(args.size() + asz);
-            fill_aligned_energy_args(args.data() + args.size() - asz, VSig{s.deg, 0, (int64_t)s.dl, (int64_t)s.dl},
-                                     (int64_t)s.rl, d_lags + i, s.stats + 8, s.lag_job ? s.stats + 4 : nullptr);
-            ++na;
+            jobs.push_back(AlignedEnergyJob{VSig{s.deg, 0, (int64_t)s.dl, (int64_t)s.dl}, (int64_t)s.rl, d_lags + i,
+                                            s.stats + 8, s.lag_job ? s.stats + 4 : nullptr});
+            max_len = std::max(max_len, (int64_t)s.dl);
         }
-        if (na && opt_.form != kFormExact)
-            launch_aligned_energy_tree(upload_bytes(args.data(), args.size()), na,
-                                       arena_.alloc_n<double>((size_t)na * kTreeParts * 3), stream_);
-        else if (na)
-            launch_aligned_energy(upload_bytes(args.data(), args.size()), na, stream_);
+        if (jobs.empty()) return;
+        const int na = (int)jobs.size();
+        if (opt_.form != kFormExact)
+            launch_aligned_energy_tree(upload(jobs), na, arena_.alloc_n<double>((size_t)na * kTreeParts * 3), stream_);
+        else
+            launch_aligned_energy(upload(jobs), na, max_len, arena_.alloc(serial_sum_scratch(na, max_len)), stream_);
     };
     {
         std::vector<SumJob> sums;

@@ -206,6 +206,7 @@ private:
     };
     // Envelope statistics of sum jobs: serial (exact) or tree (fast).
     void launch_sums(const std::vector<SumJob> &sums);
+    void launch_serial_sums(const std::vector<SumJob> &sums);
     // The launch shape for a kernel class among candidates: measured on the
     // caller's jobs at first use per device (launch(c) launches them with
     // shape c on st), then reused; candidates[0] when autotuning is off.

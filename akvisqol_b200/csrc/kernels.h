@@ -75,16 +75,18 @@ enum Form : int32_t {
 // Kernels launched by this thread so far (each launcher counts its own).
 uint64_t &launch_counter();
 
+// k_sums.cu: sums in the CPU's order, every rounding reproduced. max_len: the
+// longest signal of the jobs; d_scratch: serial_sum_scratch(njobs, max_len)
+// bytes at a 256-byte boundary.
+size_t serial_sum_scratch(int njobs, int64_t max_len);
+void launch_envelope_stats(const SumJob *d_jobs, int njobs, int64_t max_len, void *d_scratch, cudaStream_t s);
+void launch_energy(const SumJob *d_jobs, int njobs, int64_t max_len, void *d_scratch, cudaStream_t s);
+// deg_stats of a job: launch_envelope_stats's sums of the whole degraded
+// signal, from which the aligned energy is taken when the lag drops only
+// zero terms; or null.
+void launch_aligned_energy(const AlignedEnergyJob *d_jobs, int njobs, int64_t max_len, void *d_scratch, cudaStream_t s);
+
 // k_signal.cu
-void launch_envelope_stats(const SumJob *d_jobs, int njobs, cudaStream_t s);
-void launch_energy(const SumJob *d_jobs, int njobs, cudaStream_t s);
-size_t aligned_energy_args_size();
-// d_deg_stats: the exact form's serial sums of the whole degraded signal
-// (launch_envelope_stats), from which the aligned energy is taken when the
-// lag drops only zero terms; or null.
-void fill_aligned_energy_args(void *dst, const VSig &deg, int64_t ref_len, const int64_t *d_lag, double *d_out,
-                              const double *d_deg_stats = nullptr);
-void launch_aligned_energy(const void *d_args, int njobs, cudaStream_t s);
 void launch_pack(const LagJob *d_jobs, int njobs, int64_t max_n, bool raw, cudaStream_t s);
 size_t scale_args_size();
 void fill_scale_args(void *dst, const VSig &src, double factor, double *out);
@@ -94,7 +96,7 @@ void launch_scale(const void *d_args, int njobs, int64_t max_len, cudaStream_t s
 // scratch: kTreeParts * 3 doubles per job.
 constexpr int kTreeParts = 32;
 void launch_envelope_stats_tree(const SumJob *d_jobs, int njobs, double *d_scratch, cudaStream_t s);
-void launch_aligned_energy_tree(const void *d_args, int njobs, double *d_scratch, cudaStream_t s);
+void launch_aligned_energy_tree(const AlignedEnergyJob *d_jobs, int njobs, double *d_scratch, cudaStream_t s);
 
 // k_fft.cu
 void fft_init_attributes();

@@ -119,8 +119,9 @@ int visqol_b200_signal_sums(const double *x, size_t len, size_t skip, double *ou
         // x[skip..] as a window: sample(i) = x[i + skip]
         const vqb::SumJob tail{vqb::VSig{dx.p, -k, n, n - k}, dout.p + 4};
         DBuf<vqb::SumJob> dw(&whole, 1), dt(&tail, 1);
-        vqb::launch_envelope_stats(dw.p, 1, 0);
-        vqb::launch_energy(dt.p, 1, 0);
+        DBuf<char> scratch(vqb::serial_sum_scratch(1, n));
+        vqb::launch_envelope_stats(dw.p, 1, n, scratch.p, 0);
+        vqb::launch_energy(dt.p, 1, n, scratch.p, 0);
         VQB_CUDA(cudaDeviceSynchronize());
         double h[8];
         dout.get(h, 8);

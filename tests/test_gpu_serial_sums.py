@@ -112,3 +112,26 @@ def test_bench_signals(native, kind):
         ref, deg = synth.speech_pair(synth.SEED_BASE + 0x8000, seconds=8.0)
     check(native, ref, skip=1778)
     check(native, deg, skip=1778)
+
+
+def segment_case(kind, n):
+    """Signals that strain the segmented sums: 16-bit samples (alternating
+    sums next to powers of two), a level that jumps by 2^12 inside a segment
+    (sums that leave the binades their start allows for), and a sum that
+    sits on a binade's edge."""
+    rng = np.random.default_rng(n + len(kind))
+    if kind == "pcm":
+        return np.round(rng.standard_normal(n) * 2000) / 32768.0
+    if kind == "jumps":
+        return rng.standard_normal(n) * 0.1 * 2.0 ** (-12.0 * ((np.arange(n) // 700) % 2))
+    x = np.zeros(n)
+    x[0] = 1.0
+    x[1:] = np.where(np.arange(n - 1) % 2, -1.0, 1.0) * 2.0 ** -53 * rng.integers(0, 3, n - 1)
+    return x
+
+
+# segments are 256, 512, 1024 and 2048 samples long below 2^16, 2^18, 2^21 and above
+@pytest.mark.parametrize("kind", ["pcm", "jumps", "edge"])
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 319, 513, 1025, 8191, 65535, 65537, (1 << 18) - 1, 1 << 18, (1 << 21) + 77])
+def test_segments(native, kind, n):
+    check(native, segment_case(kind, n), skip=min(n, 1000))
