@@ -488,10 +488,12 @@ uint64_t Engine::launch_spectrograms(const std::vector<SpecJob> &jobs, const Rat
         if (begin) VQB_CUDA(cudaEventRecord(begin, st));
         launch(shape);
     } else {
-        const int F = tuned(kTuneGammatone, opt_.form, nbi,
-                            opt_.form == kFormF64 ? gammatone_f64fma_frames_candidates(nbi)
-                                                  : gammatone_frames_candidates(nbi),
-                            launch_frames, st);
+        // exact form: a rule's shape (VISQOL_TUNE_0 may fix another)
+        const std::vector<int> shapes = gammatone_frames_shapes(nbi);
+        const int F = opt_.form == kFormF64
+                          ? tuned(kTuneGammatone, opt_.form, nbi, gammatone_f64fma_frames_candidates(nbi),
+                                  launch_frames, st)
+                          : tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, launch_frames, st, &shapes);
         if (opt_.form == kFormF64) {
             // the FP64-FMA kernel at that shape, or the same form on the FP32
             // kernel's staged tiles (same bits); tile lists uploaded on first use

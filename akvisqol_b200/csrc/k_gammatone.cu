@@ -4,11 +4,20 @@
 // Every (frame, band) RMS is an independent 4-biquad recurrence over one
 // Hann-windowed frame from zero state, so one thread owns one (frame, band)
 // and keeps the eight state values in registers. A CTA takes F consecutive
-// frames of one job with all NB bands (F = 256 / NB: 8 frames for 32 bands,
-// 12 for 21); in a warp the lanes read the same or neighbouring samples,
-// which L1 serves as a broadcast, and the Hann value is uniform across the
-// CTA. The work is FP64-pipe bound: 31 dependent-chain f64 operations per
-// sample (no FMA, as the CPU), 1 load of signal and 1 of window.
+// frames of one job with all NB bands (thread = frame * NB + band) and stages
+// their windowed samples, each product formed once, in shared memory 64 at a
+// time; the next 64 are loaded into registers meanwhile.
+//
+// The work is FP64-pipe bound: 30 separately rounded f64 operations a sample
+// (no FMA, as the CPU), 60 issue cycles of a warp's scheduler. The four
+// biquads run skewed, stage k on sample i - k, so that a step holds four
+// independent recurrences instead of one chain through all of them: the same
+// operations on the same operands. That matters where a scheduler has one
+// warp (a single pair's spectrogram is 500 warps on 592 schedulers): with the
+// staging, 295 -> 173 us for 10 s at 48 kHz and 149 -> 65 us for 2.5 s of
+// speech, against 122 and 41 us of pure issue.
+#include <algorithm>
+
 #include "device.cuh"
 #include "kernels.h"
 
@@ -21,55 +30,97 @@ struct Tile {
     int32_t frame0;
 };
 
+constexpr int kTileS = 64;        // samples staged at a time
+constexpr int kRow = kTileS + 2;  // a frame's row of a stage (rows of a warp in different banks)
+
+// Transposed direct form II with the CPU's operation order.
+struct Biquad {
+    double c0 = 0.0, c1 = 0.0;
+    __device__ inline double step(double x, double n0, double n1, double d1, double d2) {
+        const double y = n0 * x + c0;
+        c0 = n1 * x + c1 - d1 * y;
+        c1 = -(d2 * y);
+        return y;
+    }
+};
+
+// wx: [2][frames][kRow] windowed samples (dynamic shared memory).
 __global__ void __launch_bounds__(256) gammatone_kernel(const SpecJob *__restrict__ jobs, const Tile *__restrict__ tiles,
                                                         const BandCoeffs *__restrict__ coeffs, int nb,
                                                         const double *__restrict__ hann, int window, int hop) {
+    extern __shared__ __align__(16) double wx[];
     const Tile tile = tiles[blockIdx.x];
-    const int frames_per_cta = blockDim.x / nb;
+    const int frames = blockDim.x / nb;
     const int fl = threadIdx.x / nb;
     const int band = threadIdx.x - fl * nb;
-    if (fl >= frames_per_cta) return;
     const SpecJob job = jobs[tile.job];
+    const VSig sig = job.sig;
+    const BandCoeffs k = coeffs[band];
+    const int total = frames * kTileS;
+    // entry e of a tile: frame e / kTileS, sample e % kTileS. A thread holds
+    // its entries' samples of the next tile in registers (64 / nb of them, at
+    // most kHold), the rest are loaded when they are windowed.
+    constexpr int kHold = 4;
+    double held[kHold];
+    auto sample = [&](int e, int i0) {
+        const int c = e / kTileS, i = i0 + (e - c * kTileS);
+        return i < window ? vsig_at(sig, ((int64_t)tile.frame0 + c) * hop + i) : 0.0;
+    };
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int m = 0; m < kHold; ++m) {
+            const int e = threadIdx.x + m * blockDim.x;
+            if (e < total) held[m] = sample(e, i0);
+        }
+    };
+    auto store = [&](int i0, int buf) {
+        double *w = wx + buf * frames * kRow;
+        auto put = [&](int e, double x) {
+            const int c = e / kTileS, j = e - c * kTileS, i = i0 + j;
+            w[c * kRow + j] = i < window ? x * __ldg(hann + i) : 0.0;
+        };
+#pragma unroll
+        for (int m = 0; m < kHold; ++m) {
+            const int e = threadIdx.x + m * blockDim.x;
+            if (e < total) put(e, held[m]);
+        }
+        for (int e = threadIdx.x + kHold * blockDim.x; e < total; e += blockDim.x) put(e, sample(e, i0));
+    };
+    Biquad s1, s2, s3, s4;
+    double y1 = 0.0, y2 = 0.0, y3 = 0.0, sum_sq = 0.0;
+    auto step = [&](double x) {
+        const double y4 = s4.step(y3, k.ca0, k.s4n1, k.d1, k.d2);
+        y3 = s3.step(y2, k.ca0, k.s3n1, k.d1, k.d2);
+        y2 = s2.step(y1, k.ca0, k.s2n1, k.d1, k.d2);
+        y1 = s1.step(x, k.s1n0, k.s1n1, k.d1, k.d2);
+        sum_sq += y4 * y4;
+    };
+    load(0);
+    store(0, 0);
+    load(kTileS);
+    __syncthreads();
+    int buf = 0;
+    for (int i0 = 0; i0 < window; i0 += kTileS, buf ^= 1) {
+        const double *w = wx + (buf * frames + fl) * kRow;
+        if (window - i0 >= kTileS) {
+#pragma unroll 4
+            for (int i = 0; i < kTileS; i += 2) {
+                const double2 x = *reinterpret_cast<const double2 *>(w + i);
+                step(x.x);
+                step(x.y);
+            }
+        } else {
+            for (int i = 0; i < window - i0; ++i) step(w[i]);
+        }
+        if (i0 + kTileS < window) {
+            store(i0 + kTileS, buf ^ 1);
+            if (i0 + 2 * kTileS < window) load(i0 + 2 * kTileS);
+        }
+        __syncthreads();
+    }
+    for (int i = 0; i < 3; ++i) step(0.0);  // the last three samples through the later stages
     const int64_t f = (int64_t)tile.frame0 + fl;
     if (f >= job.nf) return;
-    const BandCoeffs k = coeffs[band];
-    double s1c0 = 0, s1c1 = 0, s2c0 = 0, s2c1 = 0, s3c0 = 0, s3c1 = 0, s4c0 = 0, s4c1 = 0;
-    double sum_sq = 0;
-    const int64_t k0 = f * hop;
-    const VSig sig = job.sig;
-    auto step = [&](double s) {
-        const double f1 = k.s1n0 * s + s1c0;
-        s1c0 = k.s1n1 * s + s1c1 - k.d1 * f1;
-        s1c1 = -(k.d2 * f1);
-        const double f2 = k.ca0 * f1 + s2c0;
-        s2c0 = k.s2n1 * f1 + s2c1 - k.d1 * f2;
-        s2c1 = -(k.d2 * f2);
-        const double f3 = k.ca0 * f2 + s3c0;
-        s3c0 = k.s3n1 * f2 + s3c1 - k.d1 * f3;
-        s3c1 = -(k.d2 * f3);
-        const double f4 = k.ca0 * f3 + s4c0;
-        s4c0 = k.s4n1 * f3 + s4c1 - k.d1 * f4;
-        s4c1 = -(k.d2 * f4);
-        sum_sq += f4 * f4;
-    };
-    if (nb == 32) {
-        // A warp is one frame's 32 bands: lane j forms windowed sample
-        // i0 + j once (coalesced loads, one multiply per 32 samples) and the
-        // warp reads it by shuffle, taking the product off the FP64 pipe.
-        const int lane = threadIdx.x & 31;
-        int i0 = 0;
-        for (; i0 + 32 <= window; i0 += 32) {
-            const double x = vsig_at(sig, k0 + i0 + lane) * __ldg(hann + i0 + lane);
-#pragma unroll 8
-            for (int j = 0; j < 32; ++j) step(__shfl_sync(0xffffffffu, x, j));
-        }
-        const int rest = window - i0;
-        const double x = lane < rest ? vsig_at(sig, k0 + i0 + lane) * __ldg(hann + i0 + lane) : 0.0;
-        for (int j = 0; j < rest; ++j) step(__shfl_sync(0xffffffffu, x, j));
-    } else {
-#pragma unroll 4
-        for (int i = 0; i < window; ++i) step(vsig_at(sig, k0 + i) * __ldg(hann + i));
-    }
     const double inv_n = 1.0 / (double)window;
     job.out[(int64_t)band * job.nf + f] = sqrt(sum_sq * inv_n);
 }
@@ -87,13 +138,16 @@ __global__ void __launch_bounds__(256) copy_frames_kernel(const CopyJob *__restr
 
 }  // namespace
 
-int gammatone_frames_per_cta(int nb) { return 256 / nb; }
+// 128 threads: one warp a scheduler, and a few CTAs an SM in a large launch.
+// Measured against 256, 64 and 32 threads (spectrogram kernels of a pass, us):
+// one 10 s 48 kHz pair 519 (844, 518, 552), one 2.5 s speech pair 130 (204,
+// 133, 153), 32 10 s pairs level.
+int gammatone_frames_per_cta(int nb) { return std::max(1, std::min(128 / nb, 16)); }
 
-std::vector<int> gammatone_frames_candidates(int nb) {
-    const int f = 256 / nb;
-    std::vector<int> c{f};
+std::vector<int> gammatone_frames_shapes(int nb) {
+    const int f = gammatone_frames_per_cta(nb);
+    std::vector<int> c{f, 2 * f};
     if (f / 2 >= 1) c.push_back(f / 2);
-    if (f / 4 >= 1) c.push_back(f / 4);
     return c;
 }
 size_t gammatone_tile_size() { return sizeof(Tile); }
@@ -103,7 +157,8 @@ void launch_gammatone(const SpecJob *d_jobs, const void *d_tiles, int ntiles, co
                       const double *d_hann, int window, int hop, int frames_per_cta, cudaStream_t s) {
     if (ntiles <= 0) return;
     const int threads = frames_per_cta * nb;
-    gammatone_kernel<<<ntiles, threads, 0, s>>>(d_jobs, static_cast<const Tile *>(d_tiles), d_coeffs, nb, d_hann,
+    const size_t smem = (size_t)2 * frames_per_cta * kRow * sizeof(double);
+    gammatone_kernel<<<ntiles, threads, smem, s>>>(d_jobs, static_cast<const Tile *>(d_tiles), d_coeffs, nb, d_hann,
                                                window, hop);
     launch_counter() += 1;
 }

@@ -150,9 +150,7 @@ void launch_refine_approx(const LagJob *d_job, int64_t n, int nchunks, cudaStrea
 
 // k_gammatone.cu
 int gammatone_frames_per_cta(int nb);
-// CTA shapes the autotuner may choose among for the exact and FP64 FMA
-// kernels (frames per CTA; the first is the default).
-std::vector<int> gammatone_frames_candidates(int nb);
+std::vector<int> gammatone_frames_shapes(int nb);  // all valid frames per CTA, the rule's first
 size_t gammatone_tile_size();
 void fill_gammatone_tile(void *dst, int job, int frame0);
 void launch_gammatone(const SpecJob *d_jobs, const void *d_tiles, int ntiles, const BandCoeffs *d_coeffs, int nb,

@@ -28,6 +28,20 @@ def test_spectrogram_bit_identical(native, oracle, nb, sr, frames):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("nb", [1, 5, 8, 31, 32])
+@pytest.mark.parametrize("window,frames", [(1, 1), (3, 5), (63, 17), (64, 4), (65, 2), (130, 33)])
+def test_spectrogram_tile_edges(native, oracle, nb, window, frames):
+    """Windows around the kernel's 64-sample tiles and the three samples its
+    skewed stages hold, and band and frame counts that leave CTAs partly
+    filled: the CPU's bits."""
+    coeffs, _ = oracle.filters(nb, 48000, 50.0, 24000.0)
+    hop = max(1, window // 4)
+    x = np.random.default_rng(window * 100 + nb).uniform(-1, 1, window + (frames - 1) * hop)
+    got = native.spectrogram(x, coeffs, oracle.hann(window), window, hop)
+    want = oracle.spectrogram(x, coeffs, window, hop)
+    assert np.array_equal(got, want)
+
+
 def test_spectrogram_full_pair(native, oracle, audio0):
     ref, _ = audio0
     coeffs, _ = oracle.filters(32, 48000)
