@@ -357,7 +357,7 @@ bool run_lanes_queued(visqol_ctx *c, size_t n, const double *const *refs, const 
             VQB_CUDA(cudaStreamWaitEvent(e.stream(), st.chunk_done[k], 0));
             const size_t b0 = bounds[k], m = bounds[k + 1] - b0;
             e.measure_batch(m, d_ref.data() + b0, ref_lens + b0, d_deg.data() + b0, deg_lens + b0, sample_rate,
-                            true, part, prepared ? prepared + b0 : nullptr, refs + b0);
+                            true, part, prepared ? prepared + b0 : nullptr);
             for (size_t j = 0; j < m; ++j) res[b0 + j] = std::move(part[j]);
             add_batch_timing(lane_t[l], e.last_timing());
         } catch (...) {
@@ -409,7 +409,7 @@ void run_lanes(visqol_ctx *c, size_t n, const double *const *refs, const size_t 
         if (streamed)
             e.measure_batch_streamed(m, r, rl, d, dl, sample_rate, o, pr);
         else
-            e.measure_batch(m, r, rl, d, dl, sample_rate, device_inputs, o, pr, nullptr, grads);
+            e.measure_batch(m, r, rl, d, dl, sample_rate, device_inputs, o, pr, grads);
     };
     if (L <= 1) {
         measure(*c->lanes[0], n, refs, ref_lens, degs, deg_lens, res, prepared);

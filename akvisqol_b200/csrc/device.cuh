@@ -126,6 +126,15 @@ __host__ __device__ inline void aligned_range(const AlignedEnergyJob &job, int64
     }
 }
 
+// Speech-mode VAD of one reference (reference src/vad.zig:15-81): loud[c] = 1
+// where the RMS of the int16-scaled samples [first + c frame_len,
+// first + (c + 1) frame_len) reaches 5000, c < chunks.
+struct VadJob {
+    VSig sig;
+    int32_t chunks, first, frame_len;
+    uint8_t *loud;
+};
+
 // One spectrogram pair to prepare for comparison (reference
 // src/spectrogram.zig:69-80): in-place on ref[nb*nfr], deg[nb*nfd].
 struct PrepJob {

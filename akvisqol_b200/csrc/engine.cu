@@ -49,6 +49,7 @@ void cuda_check(cudaError_t e, const char *what) {
 // Arenas
 // ---------------------------------------------------------------------------
 namespace {
+constexpr double kVadOverlap = 0.25;  // VAD chunk over analysis window
 constexpr size_t kAlign = 256;
 constexpr size_t kChunk = size_t(256) << 20;
 inline size_t round_up(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
@@ -269,13 +270,36 @@ T *Engine::upload(const std::vector<T> &v) {
     return static_cast<T *>(upload_bytes(v.data(), v.size() * sizeof(T)));
 }
 
+// Small uploads (job arrays) are gathered: each takes a place in a page-locked
+// chunk and the same place in a device chunk, and flush_uploads sends what is
+// pending in one copy, before the first launch that reads any of it.
 void *Engine::upload_bytes(const void *src, size_t bytes) {
-    void *h = pinned_.alloc(bytes);
-    if (bytes) std::memcpy(h, src, bytes);
-    void *d = arena_.alloc(bytes);
-    if (bytes) VQB_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, stream_));
-    timing_.h2d_bytes += bytes;
+    const size_t need = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
+    if (up_end_ + need > up_cap_) {
+        flush_uploads();
+        up_cap_ = std::max(need, size_t(1) << 20);
+        up_host_ = static_cast<char *>(pinned_.alloc(up_cap_));
+        up_dev_ = static_cast<char *>(arena_.alloc(up_cap_));
+        up_begin_ = up_end_ = 0;
+    }
+    if (bytes) std::memcpy(up_host_ + up_end_, src, bytes);
+    void *d = up_dev_ + up_end_;
+    up_end_ += need;
     return d;
+}
+
+void Engine::flush_uploads() {
+    if (up_end_ == up_begin_) return;
+    const size_t bytes = up_end_ - up_begin_;
+    VQB_CUDA(cudaMemcpyAsync(up_dev_ + up_begin_, up_host_ + up_begin_, bytes, cudaMemcpyHostToDevice, stream_));
+    timing_.h2d_bytes += bytes;
+    up_begin_ = up_end_;
+}
+
+void Engine::begin_batch() {
+    arena_.reset();
+    pinned_.reset();
+    up_cap_ = up_begin_ = up_end_ = 0;
 }
 
 void Engine::d2h(void *dst, const void *src, size_t bytes) {
@@ -305,18 +329,13 @@ uint64_t lag_search_bytes(const LagJob &j, bool f32) {
     return f32 ? 2 * sig + 4 * 8 * (uint64_t)j.n : sig + 4 * 16 * (uint64_t)j.n;
 }
 
-int32_t *Engine::launch_lag_jobs(std::vector<LagJob> &jobs, bool raw, bool exact) {
-    if (jobs.empty()) return nullptr;
+Engine::Launches Engine::plan_lag_jobs(const std::vector<LagJob> &jobs, bool raw, int32_t *d_status) {
+    Launches launches;
     // Group by FFT size; bound each submission's buffer.
     std::map<int64_t, std::vector<size_t>> groups;
     for (size_t i = 0; i < jobs.size(); ++i) groups[jobs[i].n].push_back(i);
     const size_t budget = size_t(4) << 30;
-    const bool f32 = !exact && !opt_.exact_lag_search;
-    int32_t *d_status = nullptr;
-    if (f32) {
-        d_status = arena_.alloc_n<int32_t>(jobs.size());
-        launch_zero(d_status, jobs.size() * sizeof(int32_t), stream_);
-    }
+    const bool f32 = d_status != nullptr;
     for (auto &g : groups) {
         const int64_t n = g.first;
         const Twiddles tw = twiddles((size_t)n);
@@ -349,20 +368,22 @@ int32_t *Engine::launch_lag_jobs(std::vector<LagJob> &jobs, bool raw, bool exact
                     j.rescore = rescore + (size_t)kLagCandCap * nchunks * k;
                     chunk[k] = j;
                 }
-                LagJob *d_chunk = upload(chunk);
-                auto launch32 = [&](int columns) {
-                    launch_lag32(d_chunk, (int)cnt, n, raw, tw.cols32, tw.block32, tw.stages32, nchunks, columns,
-                                 stream_);
-                };
-                // forward samples staged in shared memory, or loaded into
-                // registers: measured per transform size
-                const char *env = std::getenv("VISQOL_LAG_COLUMNS");
-                const int columns = !fused_lag_register_columns(n) ? 0
-                                    : env && (env[0] == '0' || env[0] == '1' || env[0] == '2')
-                                        ? env[0] - '0'
-                                        : tuned(kTuneLagColumns, (int)std::log2((double)n), raw ? 3 : 2, {2, 1},
-                                                launch32, stream_);
-                launch32(columns);
+                const LagJob *d_chunk = upload(chunk);
+                launches.push_back([=] {
+                    auto launch32 = [&](int columns) {
+                        launch_lag32(d_chunk, (int)cnt, n, raw, tw.cols32, tw.block32, tw.stages32, nchunks, columns,
+                                     stream_);
+                    };
+                    // forward samples staged in shared memory, or loaded into
+                    // registers: measured per transform size
+                    const char *env = std::getenv("VISQOL_LAG_COLUMNS");
+                    const int columns = !fused_lag_register_columns(n) ? 0
+                                        : env && (env[0] == '0' || env[0] == '1' || env[0] == '2')
+                                            ? env[0] - '0'
+                                            : tuned(kTuneLagColumns, (int)std::log2((double)n), raw ? 3 : 2, {2, 1},
+                                                    launch32, stream_);
+                    launch32(columns);
+                });
                 continue;
             }
             // (above 2^24 points the exact search decides in every form; status stays 0)
@@ -372,39 +393,48 @@ int32_t *Engine::launch_lag_jobs(std::vector<LagJob> &jobs, bool raw, bool exact
                 chunk[k] = jobs[g.second[c0 + k]];
                 chunk[k].z = z + (int64_t)k * n;
             }
-            LagJob *d_jobs = upload(chunk);
+            const LagJob *d_jobs = upload(chunk);
             if (fused_lag_supported(n)) {
                 const size_t parts = fused_lag_parts(n);
                 double *pv = arena_.alloc_n<double>(parts * cnt);
                 int64_t *pk = arena_.alloc_n<int64_t>(parts * cnt);
-                auto launch = [&](int columns) {
-                    launch_fused_lag(d_jobs, (int)cnt, n, raw, tw.cols, tw.block, tw.stages, pv, pk, columns, stream_);
-                };
-                // column passes: shared-memory tiles, registers, or registers
-                // with the forward samples staged, measured per transform size
-                // (VISQOL_LAG_COLUMNS=0/1/2 fixes the choice)
-                int columns = 0;
-                if (fused_lag_register_columns(n)) {
-                    const char *env = std::getenv("VISQOL_LAG_COLUMNS");
-                    columns = env && (env[0] == '0' || env[0] == '1' || env[0] == '2')
-                                  ? env[0] - '0'
-                                  : tuned(kTuneLagColumns, (int)std::log2((double)n), raw ? 1 : 0, {1, 2, 0},
-                                          launch, stream_);
-                }
-                launch(columns);
+                launches.push_back([=] {
+                    auto launch = [&](int columns) {
+                        launch_fused_lag(d_jobs, (int)cnt, n, raw, tw.cols, tw.block, tw.stages, pv, pk, columns, stream_);
+                    };
+                    // column passes: shared-memory tiles, registers, or registers
+                    // with the forward samples staged, measured per transform size
+                    // (VISQOL_LAG_COLUMNS=0/1/2 fixes the choice)
+                    int columns = 0;
+                    if (fused_lag_register_columns(n)) {
+                        const char *env = std::getenv("VISQOL_LAG_COLUMNS");
+                        columns = env && (env[0] == '0' || env[0] == '1' || env[0] == '2')
+                                      ? env[0] - '0'
+                                      : tuned(kTuneLagColumns, (int)std::log2((double)n), raw ? 1 : 0, {1, 2, 0},
+                                              launch, stream_);
+                    }
+                    launch(columns);
+                });
                 continue;
             }
             const int parts = argmax_parts(n);
             double *pv = arena_.alloc_n<double>((size_t)parts * cnt);
             int64_t *pk = arena_.alloc_n<int64_t>((size_t)parts * cnt);
-            launch_pack(d_jobs, (int)cnt, n, raw, stream_);
-            launch_fft(z, n, false, tw.top, tw.block, (int)cnt, n, stream_);
-            launch_cross(z, n, (int)cnt, n, stream_);
-            launch_fft(z, n, true, tw.top, tw.block, (int)cnt, n, stream_);
-            launch_argmax(z, d_jobs, (int)cnt, n, n, pv, pk, stream_);
+            launches.push_back([=] {
+                launch_pack(d_jobs, (int)cnt, n, raw, stream_);
+                launch_fft(z, n, false, tw.top, tw.block, (int)cnt, n, stream_);
+                launch_cross(z, n, (int)cnt, n, stream_);
+                launch_fft(z, n, true, tw.top, tw.block, (int)cnt, n, stream_);
+                launch_argmax(z, d_jobs, (int)cnt, n, n, pv, pk, stream_);
+            });
         }
     }
-    return d_status;
+    return launches;
+}
+
+void Engine::run(const Launches &launches) {
+    flush_uploads();
+    for (const auto &f : launches) f();
 }
 
 std::vector<size_t> Engine::rerun_undecided(const std::vector<LagJob> &jobs, const int32_t *h_status, bool raw) {
@@ -413,7 +443,7 @@ std::vector<size_t> Engine::rerun_undecided(const std::vector<LagJob> &jobs, con
     std::vector<LagJob> rerun;
     for (size_t i = 0; i < jobs.size(); ++i)
         if (h_status[i]) idx.push_back(i), rerun.push_back(jobs[i]);
-    if (!rerun.empty()) launch_lag_jobs(rerun, raw, true);
+    run(plan_lag_jobs(rerun, raw, nullptr));
     timing_.lag_reruns += idx.size();
     return idx;
 }
@@ -440,92 +470,93 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
     return b;
 }
 
-uint64_t Engine::launch_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, cudaStream_t st,
-                                     cudaEvent_t begin, cudaEvent_t end) {
-    if (jobs.empty()) return 0;
+// Tiles of F frames of the jobs.
+const void *Engine::upload_tiles(const std::vector<SpecJob> &jobs, int F, int *ntiles) {
+    const size_t tsz = gammatone_tile_size();
+    std::vector<char> tiles;
+    *ntiles = 0;
+    for (size_t j = 0; j < jobs.size(); ++j)
+        for (int64_t f = 0; f < jobs[j].nf; f += F, ++*ntiles) {
+            tiles.resize(tiles.size() + tsz);
+            fill_gammatone_tile(tiles.data() + tiles.size() - tsz, (int)j, (int)f);
+        }
+    return upload_bytes(tiles.data(), tiles.size());
+}
+
+Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc) {
+    SpecPlan plan;
+    plan.jobs = jobs;
+    plan.d_jobs = upload(jobs);
+    for (const SpecJob &j : jobs) plan.rms += (uint64_t)j.nf * nb_;
+    const int nbi = (int)nb_;
+    if (opt_.form == kFormExact) {
+        // a rule's shape (VISQOL_TUNE_0 may fix another)
+        const std::vector<int> shapes = gammatone_frames_shapes(nbi);
+        plan.frames = tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, [](int) {}, stream_, &shapes);
+    } else {
+        plan.frames = gammatone_fast_frames_per_cta();
+    }
+    plan.d_tiles = upload_tiles(jobs, plan.frames, &plan.ntiles);
+    plan.rc = &rc;
+    return plan;
+}
+
+void Engine::run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin, cudaEvent_t end) {
+    if (plan.jobs.empty()) return;
+    const RateCache &rc = *plan.rc;
+    const SpecJob *d_jobs = plan.d_jobs;
     const int nbi = (int)nb_;
     const int W = (int)rc.geo.window, H = (int)rc.geo.hop;
-    SpecJob *d_jobs = upload(jobs);
-    uint64_t rms = 0;
-    for (const SpecJob &j : jobs) rms += (uint64_t)j.nf * nb_;
-    // Tiles of F frames (the FP32 kernel's shape is fixed), uploaded on the
-    // main stream; a side stream waits for them.
-    auto tiles_of = [&](int F, int *ntiles) {
-        const size_t tsz = gammatone_tile_size();
-        std::vector<char> tiles;
-        *ntiles = 0;
-        for (size_t j = 0; j < jobs.size(); ++j)
-            for (int64_t f = 0; f < jobs[j].nf; f += F, ++*ntiles) {
-                tiles.resize(tiles.size() + tsz);
-                fill_gammatone_tile(tiles.data() + tiles.size() - tsz, (int)j, (int)f);
-            }
-        void *d = upload_bytes(tiles.data(), tiles.size());
+    // uploads go up on the main stream; a side stream waits for them
+    auto uploaded = [&] {
+        flush_uploads();
         if (st != stream_) {
             record(ev_inputs_);
             VQB_CUDA(cudaStreamWaitEvent(st, ev_inputs_, 0));
         }
-        return d;
     };
-    auto launch_frames = [&](int F) {
-        int ntiles = 0;
-        const void *d_tiles = tiles_of(F, &ntiles);
-        if (opt_.form == kFormF64)
-            launch_gammatone_f64fma(d_jobs, d_tiles, ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, F, st);
-        else
-            launch_gammatone(d_jobs, d_tiles, ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, F, st);
-    };
+    uploaded();
     if (opt_.form == kFormF32) {
-        int ntiles = 0;
-        const void *d_tiles = tiles_of(gammatone_fast_frames_per_cta(), &ntiles);
         int *queue = arena_.alloc_n<int>(1);  // the persistent form's work counter
         auto launch = [&](int shape) {
             if (shape >= 100) launch_zero(queue, sizeof(int), st);
-            launch_gammatone_fast(d_jobs, d_tiles, ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, shape, queue, st);
+            launch_gammatone_fast(d_jobs, plan.d_tiles, plan.ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, shape, queue,
+                                  st);
         };
         static const std::vector<int> all_shapes = gammatone_fast_shapes();
         const int shape =
             tuned(kTuneGammatoneFastCtas, opt_.form, nbi, gammatone_fast_shape_candidates(), launch, st, &all_shapes);
         if (begin) VQB_CUDA(cudaEventRecord(begin, st));
         launch(shape);
-    } else {
-        // exact form: a rule's shape (VISQOL_TUNE_0 may fix another)
-        const std::vector<int> shapes = gammatone_frames_shapes(nbi);
-        const int F = opt_.form == kFormF64
-                          ? tuned(kTuneGammatone, opt_.form, nbi, gammatone_f64fma_frames_candidates(nbi),
-                                  launch_frames, st)
-                          : tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, launch_frames, st, &shapes);
-        if (opt_.form == kFormF64) {
-            // the FP64-FMA kernel at that shape, or the same form on the FP32
-            // kernel's staged tiles (same bits); tile lists uploaded on first use
-            int ntiles[2] = {0, 0};
-            const void *d_tiles[2] = {nullptr, nullptr};
-            auto ensure_tiles = [&](int staged) {
-                if (!d_tiles[staged])
-                    d_tiles[staged] = tiles_of(staged ? gammatone_fast_frames_per_cta() : F, &ntiles[staged]);
-            };
-            auto launch = [&](int staged) {
-                ensure_tiles(staged);
-                if (staged)
-                    launch_gammatone_f64_staged(d_jobs, d_tiles[1], ntiles[1], rc.d_fast_coeffs, nbi, rc.d_hann, W, H,
-                                                st);
-                else
-                    launch_gammatone_f64fma(d_jobs, d_tiles[0], ntiles[0], rc.d_fast_coeffs, nbi, rc.d_hann, W, H, F,
+    } else if (opt_.form == kFormF64) {
+        // the FP64-FMA kernel at its measured shape, or the same form on the
+        // FP32 kernel's staged tiles (same bits); tile lists on first use
+        std::map<int, std::pair<const void *, int>> lists;
+        auto launch_frames = [&](int F) {
+            auto &l = lists[F];
+            if (!l.first) {
+                l.first = upload_tiles(plan.jobs, F, &l.second);
+                uploaded();
+            }
+            launch_gammatone_f64fma(d_jobs, l.first, l.second, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, F, st);
+        };
+        const int F = tuned(kTuneGammatone, opt_.form, nbi, gammatone_f64fma_frames_candidates(nbi), launch_frames, st);
+        auto launch = [&](int staged) {
+            if (staged)
+                launch_gammatone_f64_staged(d_jobs, plan.d_tiles, plan.ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H,
                                             st);
-            };
-            const int staged =
-                tuned(kTuneGammatoneF64Staged, opt_.form, nbi, gammatone_f64_staged_candidates(), launch, st);
-            ensure_tiles(staged);
-            if (begin) VQB_CUDA(cudaEventRecord(begin, st));
-            launch(staged);
-        } else {
-            int ntiles = 0;
-            const void *d_tiles = tiles_of(F, &ntiles);
-            if (begin) VQB_CUDA(cudaEventRecord(begin, st));
-            launch_gammatone(d_jobs, d_tiles, ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, F, st);
-        }
+            else
+                launch_frames(F);
+        };
+        const int staged =
+            tuned(kTuneGammatoneF64Staged, opt_.form, nbi, gammatone_f64_staged_candidates(), launch, st);
+        if (begin) VQB_CUDA(cudaEventRecord(begin, st));
+        launch(staged);
+    } else {
+        if (begin) VQB_CUDA(cudaEventRecord(begin, st));
+        launch_gammatone(d_jobs, plan.d_tiles, plan.ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, plan.frames, st);
     }
     if (end) VQB_CUDA(cudaEventRecord(end, st));
-    return rms;
 }
 
 namespace {
@@ -617,12 +648,14 @@ void Engine::prepare(size_t n, const double *const *refs, const size_t *ref_lens
                      bool device_inputs, std::vector<std::unique_ptr<PreparedRef>> &out) {
     out.clear();
     VQB_CUDA(cudaSetDevice(device_));
-    arena_.reset();
-    pinned_.reset();
+    begin_batch();
     const RateCache &rc = rate_cache(sample_rate);
     const size_t W = rc.geo.window, H = rc.geo.hop, P = patch_;
     std::vector<SumJob> sums;
     std::vector<SpecJob> specs;
+    std::vector<VadJob> vads;
+    std::vector<size_t> loud_at(n, 0);
+    size_t nloud = 0;
     for (size_t i = 0; i < n; ++i) {
         auto p = std::make_unique<PreparedRef>();
         p->device = device_;
@@ -643,11 +676,26 @@ void Engine::prepare(size_t n, const double *const *refs, const size_t *ref_lens
             const VSig sig{p->d_sig, 0, (int64_t)p->len, (int64_t)p->len};
             sums.push_back(SumJob{sig, p->d_stats});
             specs.push_back(SpecJob{sig, (int64_t)p->nf, p->d_spec});
+            if (opt_.speech) {
+                loud_at[i] = nloud;
+                vads.push_back(vad_job(sig, p->nf, W, &nloud));
+            }
         }
         out.push_back(std::move(p));
     }
-    launch_sums(sums);
-    launch_spectrograms(specs, rc, stream_);
+    uint8_t *d_loud = arena_.alloc_n<uint8_t>(std::max<size_t>(1, nloud));
+    {
+        size_t v = 0;
+        for (size_t i = 0; i < n; ++i)
+            if (opt_.speech && out[i]->d_sig) vads[v++].loud = d_loud + loud_at[i];
+    }
+    const Launches do_sums = plan_sums(sums), do_vad = plan_vad(vads);
+    const SpecPlan spec = plan_spectrograms(specs, rc);
+    run(do_sums);
+    run(do_vad);
+    run_spectrograms(spec, stream_);
+    uint8_t *h_loud = pinned_.alloc_n<uint8_t>(std::max<size_t>(1, nloud));
+    d2h(h_loud, d_loud, nloud);
     std::vector<double> h(4 * n, 0.0);
     for (size_t i = 0; i < n; ++i)
         if (out[i]->d_stats) VQB_CUDA(cudaMemcpyAsync(h.data() + 4 * i, out[i]->d_stats, 4 * sizeof(double),
@@ -658,14 +706,7 @@ void Engine::prepare(size_t n, const double *const *refs, const size_t *ref_lens
         if (p.code) continue;
         std::copy(h.begin() + 4 * i, h.begin() + 4 * i + 4, p.stats);
         if (opt_.speech) {
-            std::vector<double> tmp;
-            const double *hr = refs[i];
-            if (device_inputs) {
-                tmp.resize(p.len);
-                VQB_CUDA(cudaMemcpy(tmp.data(), refs[i], p.len * sizeof(double), cudaMemcpyDeviceToHost));
-                hr = tmp.data();
-            }
-            p.idx = host::vad_patch_indices(hr, p.len, p.nf, P, W, 0.25);
+            p.idx = host::vad_patches(h_loud + loud_at[i], p.nf, P, W, kVadOverlap);
         } else {
             p.idx = host::ref_patch_indices(p.nf, P);
         }
@@ -676,27 +717,44 @@ void Engine::prepare(size_t n, const double *const *refs, const size_t *ref_lens
     }
 }
 
-void Engine::launch_sums(const std::vector<SumJob> &sums) {
-    if (sums.empty()) return;
-    if (opt_.form == kFormExact) {
-        launch_serial_sums(sums);
-        return;
+Engine::Launches Engine::plan_sums(const std::vector<SumJob> &sums, bool serial) {
+    if (sums.empty()) return {};
+    const int n = (int)sums.size();
+    const SumJob *d = upload(sums);
+    if (!serial && opt_.form != kFormExact) {
+        double *scratch = arena_.alloc_n<double>(sums.size() * kTreeParts * 3);
+        return {[=] { launch_envelope_stats_tree(d, n, scratch, stream_); }};
     }
-    launch_envelope_stats_tree(upload(sums), (int)sums.size(), arena_.alloc_n<double>(sums.size() * kTreeParts * 3),
-                               stream_);
-}
-
-void Engine::launch_serial_sums(const std::vector<SumJob> &sums) {
     int64_t max_len = 0;
     for (const SumJob &j : sums) max_len = std::max(max_len, j.sig.len);
-    launch_envelope_stats(upload(sums), (int)sums.size(), max_len,
-                          arena_.alloc(serial_sum_scratch((int)sums.size(), max_len)), stream_);
+    void *scratch = arena_.alloc(serial_sum_scratch(n, max_len));
+    return {[=] { launch_envelope_stats(d, n, max_len, scratch, stream_); }};
+}
+
+// The VAD of a reference of nf frames; *at: chunks so far, advanced by its own.
+VadJob Engine::vad_job(const VSig &sig, size_t nf, size_t window, size_t *at) const {
+    VadJob j{};
+    j.sig = sig;
+    j.chunks = (int32_t)host::vad_chunks(nf, patch_, window, kVadOverlap);
+    j.first = (int32_t)(patch_ / 2 - 1);
+    j.frame_len = (int32_t)((double)window * kVadOverlap);
+    *at += (size_t)j.chunks;
+    return j;
+}
+
+Engine::Launches Engine::plan_vad(const std::vector<VadJob> &jobs) {
+    if (jobs.empty()) return {};
+    int max_chunks = 0;
+    for (const VadJob &j : jobs) max_chunks = std::max(max_chunks, (int)j.chunks);
+    const VadJob *d = upload(jobs);
+    const int n = (int)jobs.size();
+    double *scratch = arena_.alloc_n<double>(jobs.size() * kTreeParts);
+    return {[=] { launch_vad(d, n, max_chunks, scratch, stream_); }};
 }
 
 void Engine::lags(size_t njobs, const VSig *a, const VSig *b, bool raw, int64_t *h_lags, int32_t *status_out,
                   float *d_corr) {
-    arena_.reset();
-    pinned_.reset();
+    begin_batch();
     std::vector<LagJob> jobs(njobs);
     int64_t *d_lags = arena_.alloc_n<int64_t>(njobs);
     double *d_stats = arena_.alloc_n<double>(8 * njobs);
@@ -715,31 +773,35 @@ void Engine::lags(size_t njobs, const VSig *a, const VSig *b, bool raw, int64_t 
         sums.push_back(SumJob{b[i], j.stats_b});
     }
     VQB_CUDA(cudaMemsetAsync(d_lags, 0, njobs * sizeof(int64_t), stream_));
-    std::vector<size_t> empty;
-    std::vector<LagJob> run;
+    std::vector<LagJob> todo;
     std::vector<size_t> where;
     for (size_t i = 0; i < njobs; ++i)
-        if (jobs[i].biggest > 0) run.push_back(jobs[i]), where.push_back(i);
-    if (!raw && !sums.empty()) launch_serial_sums(sums);
-    int32_t *d_status = launch_lag_jobs(run, raw);
+        if (jobs[i].biggest > 0) todo.push_back(jobs[i]), where.push_back(i);
+    int32_t *d_status = nullptr;
+    if (!opt_.exact_lag_search) {
+        d_status = arena_.alloc_n<int32_t>(std::max<size_t>(1, todo.size()));
+        launch_zero(d_status, std::max<size_t>(1, todo.size()) * sizeof(int32_t), stream_);
+    }
+    const Launches do_sums = raw ? Launches{} : plan_sums(sums, true), do_lags = plan_lag_jobs(todo, raw, d_status);
+    run(do_sums);
+    run(do_lags);
     int64_t *h = pinned_.alloc_n<int64_t>(njobs);
-    int32_t *h_status = d_status ? pinned_.alloc_n<int32_t>(run.size()) : nullptr;
+    int32_t *h_status = d_status ? pinned_.alloc_n<int32_t>(std::max<size_t>(1, todo.size())) : nullptr;
     d2h(h, d_lags, njobs * sizeof(int64_t));
-    if (h_status && !run.empty()) d2h(h_status, d_status, run.size() * sizeof(int32_t));
+    if (h_status) d2h(h_status, d_status, todo.size() * sizeof(int32_t));
     sync();
-    if (!rerun_undecided(run, h_status, raw).empty()) {
+    if (!rerun_undecided(todo, h_status, raw).empty()) {
         d2h(h, d_lags, njobs * sizeof(int64_t));
         sync();
     }
     std::memcpy(h_lags, h, njobs * sizeof(int64_t));
     if (status_out)
-        for (size_t k = 0; k < run.size(); ++k) status_out[where[k]] = h_status ? h_status[k] : 0;
+        for (size_t k = 0; k < todo.size(); ++k) status_out[where[k]] = h_status ? h_status[k] : 0;
 }
 
 bool Engine::refine_approx(const VSig &a, const VSig &b, const float *d_approx, int64_t n, double slack,
                            double energy, int64_t *lag) {
-    arena_.reset();
-    pinned_.reset();
+    begin_batch();
     LagJob j{};
     j.a = a;
     j.b = b;
@@ -759,7 +821,9 @@ bool Engine::refine_approx(const VSig &a, const VSig &b, const float *d_approx, 
     j.rescore = arena_.alloc_n<double>((size_t)kLagCandCap * nchunks);
     j.lag_out = arena_.alloc_n<int64_t>(1);
     launch_zero(j.lag_out, sizeof(int64_t), stream_);
-    launch_refine_approx(upload(std::vector<LagJob>{j}), n, nchunks, stream_);
+    const LagJob *d_job = upload(std::vector<LagJob>{j});
+    flush_uploads();
+    launch_refine_approx(d_job, n, nchunks, stream_);
     int64_t *h = pinned_.alloc_n<int64_t>(1);
     int32_t *st = pinned_.alloc_n<int32_t>(1);
     d2h(h, j.lag_out, sizeof(int64_t));
@@ -771,22 +835,16 @@ bool Engine::refine_approx(const VSig &a, const VSig &b, const float *d_approx, 
 
 void Engine::spectrogram(const host::Filterbank &fb, const double *d_hann, size_t window, size_t hop,
                          const double *d_x, size_t len, double *d_out, size_t nf) {
-    arena_.reset();
-    pinned_.reset();
+    begin_batch();
     if (nf == 0) return;
     BandCoeffs *d_coeffs = upload(fb.run);
     SpecJob job{VSig{d_x, 0, (int64_t)len, (int64_t)len}, (int64_t)nf, d_out};
-    SpecJob *d_job = upload(std::vector<SpecJob>{job});
-    const int nbi = (int)fb.nb;
-    const int F = gammatone_frames_per_cta(nbi);
-    const size_t tsz = gammatone_tile_size();
-    std::vector<char> tiles;
+    const std::vector<SpecJob> jobs{job};
+    const SpecJob *d_job = upload(jobs);
+    const int nbi = (int)fb.nb, F = gammatone_frames_per_cta(nbi);
     int ntiles = 0;
-    for (size_t f = 0; f < nf; f += F, ++ntiles) {
-        tiles.resize(tiles.size() + tsz);
-        fill_gammatone_tile(tiles.data() + tiles.size() - tsz, 0, (int)f);
-    }
-    void *d_tiles = upload_bytes(tiles.data(), tiles.size());
+    const void *d_tiles = upload_tiles(jobs, F, &ntiles);
+    flush_uploads();
     launch_gammatone(d_job, d_tiles, ntiles, d_coeffs, nbi, d_hann, (int)window, (int)hop, F, stream_);
     sync();
 }
@@ -811,8 +869,8 @@ struct PairState {
     int code = 0;
     std::string msg;
     const double *ref = nullptr, *deg = nullptr;  // device
-    const double *h_ref = nullptr;                // host (VAD)
     size_t rl = 0, dl = 0;
+    size_t patch0 = 0;  // first patch among the batch's
     bool lag_job = false;
     double *stats = nullptr;  // device: ref[4], deg[4], aligned energy, aligned length
     host::Aligned al{};
@@ -847,8 +905,7 @@ using detail::RealignPatch;
 
 void Engine::measure_batch(size_t n, const double *const *refs, const size_t *ref_lens, const double *const *degs,
                            const size_t *deg_lens, uint32_t sample_rate, bool device_inputs,
-                           std::vector<PairOutcome> &out, const PreparedRef *const *prepared,
-                           const double *const *host_refs, bool grads) {
+                           std::vector<PairOutcome> &out, const PreparedRef *const *prepared, bool grads) {
     out.assign(n, PairOutcome{});
     timing_ = Timing{};
     if (n == 0) return;
@@ -857,8 +914,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         for (auto &o : out) o.code = kInvalid, o.message = "InvalidInput";
         return;
     }
-    arena_.reset();
-    pinned_.reset();
+    begin_batch();
     const RateCache &rc = rate_cache(sample_rate);
     const size_t W = rc.geo.window, H = rc.geo.hop, NB = nb_, P = patch_;
     const double fd = rc.geo.frame_duration;
@@ -884,7 +940,6 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         if (device_inputs) {
             s.ref = s.prep ? s.prep->d_sig : refs[i];
             s.deg = degs[i];
-            if (host_refs && !s.prep) s.h_ref = host_refs[i];
         } else {
             double *d = arena_.alloc_n<double>(s.dl);
             if (s.dl) VQB_CUDA(cudaMemcpyAsync(d, degs[i], s.dl * sizeof(double), cudaMemcpyHostToDevice, stream_));
@@ -898,55 +953,74 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
                     VQB_CUDA(cudaMemcpyAsync(r, refs[i], s.rl * sizeof(double), cudaMemcpyHostToDevice, stream_));
                 timing_.h2d_bytes += s.rl * sizeof(double);
                 s.ref = r;
-                s.h_ref = refs[i];
             }
         }
-        s.stats = arena_.alloc_n<double>(10);
     }
 
-    auto launch_prep_jobs = [&](const std::vector<PrepJob> &jobs) {
+    auto plan_prep_jobs = [&](const std::vector<PrepJob> &jobs) -> Launches {
+        if (jobs.empty()) return {};
         int max_frames = 0;
         for (const PrepJob &j : jobs) max_frames = std::max({max_frames, (int)j.nfr, (int)j.nfd});
         double *scratch = arena_.alloc_n<double>(prep_scratch_count((int)jobs.size(), max_frames));
-        launch_prep(upload(jobs), (int)jobs.size(), nbi, max_frames, scratch, stream_);
+        const PrepJob *d = upload(jobs);
+        const int count = (int)jobs.size();
+        return {[=] { launch_prep(d, count, nbi, max_frames, scratch, stream_); }};
     };
-    auto run_gammatone = [&](const std::vector<SpecJob> &jobs, cudaStream_t st) {
-        if (jobs.empty()) return;
+    auto run_gammatone = [&](const SpecPlan &plan, cudaStream_t st) {
+        if (plan.jobs.empty()) return;
         const size_t slot = 2 * timing_.gammatone_launches;
-        const uint64_t rms = launch_spectrograms(jobs, rc, st, gt_events_[slot], gt_events_[slot + 1]);
+        run_spectrograms(plan, st, gt_events_[slot], gt_events_[slot + 1]);
         timing_.gammatone_launches += 1;
-        timing_.gammatone_rms += rms;
+        timing_.gammatone_rms += plan.rms;
         timing_.gammatone_window = W;
     };
 
-    // Reference spectrograms need only the reference signal: they run on a
-    // side stream while the main stream does the serial lag-phase work.
-    {
-        std::vector<SpecJob> ref_jobs;
-        for (size_t i = 0; i < n; ++i) {
-            PairState &s = ps[i];
-            if (!s.live || s.rl <= W) continue;
-            if (s.prep) {
-                s.nf_ref = s.prep->nf;
-                s.ref_raw = s.prep->d_spec;
-                continue;
-            }
-            s.nf_ref = host::num_frames(s.rl, W, H);
-            s.ref_raw = arena_.alloc_n<double>(NB * s.nf_ref);
-            ref_jobs.push_back(SpecJob{VSig{s.ref, 0, (int64_t)s.rl, (int64_t)s.rl}, (int64_t)s.nf_ref, s.ref_raw});
-        }
-        run_gammatone(ref_jobs, side_);
-        VQB_CUDA(cudaEventRecord(ev_ref_done_, side_));
-    }
-
     // ---- 1: global lag and SPL energies --------------------------------
-    int64_t *d_lags = arena_.alloc_n<int64_t>(n);
-    launch_zero(d_lags, n * sizeof(int64_t), stream_);
+    // Reference spectrograms need only the reference signal: they run on a
+    // side stream while the main stream does the lag-phase work.
+    std::vector<SpecJob> ref_jobs;
+    std::vector<VadJob> vads;
+    std::vector<size_t> vad_at(n, SIZE_MAX);
+    size_t nloud = 0, nlag = 0;
+    for (size_t i = 0; i < n; ++i) {
+        PairState &s = ps[i];
+        if (!s.live) continue;
+        s.lag_job = !opt_.disable_global_alignment && s.rl > 0 && s.dl > 0;
+        nlag += s.lag_job;
+        if (s.rl <= W) continue;
+        if (s.prep) {
+            s.nf_ref = s.prep->nf;
+            s.ref_raw = s.prep->d_spec;
+            continue;
+        }
+        const VSig sig{s.ref, 0, (int64_t)s.rl, (int64_t)s.rl};
+        s.nf_ref = host::num_frames(s.rl, W, H);
+        s.ref_raw = arena_.alloc_n<double>(NB * s.nf_ref);
+        ref_jobs.push_back(SpecJob{sig, (int64_t)s.nf_ref, s.ref_raw});
+        if (opt_.speech) {
+            vad_at[i] = nloud;
+            vads.push_back(vad_job(sig, s.nf_ref, W, &nloud));
+        }
+    }
+    // What the host reads after this phase lies in one block: each pair's
+    // statistics (10 doubles: reference, degraded, aligned energy and length)
+    // and lag, the lag searches' status words (0: decided) and the VAD flags.
+    const size_t lags_at = 10 * n * sizeof(double), status_at = lags_at + n * sizeof(int64_t),
+                 loud_at = status_at + nlag * sizeof(int32_t), phase1_bytes = loud_at + nloud;
+    char *d_phase1 = static_cast<char *>(arena_.alloc(phase1_bytes));
+    int64_t *d_lags = reinterpret_cast<int64_t *>(d_phase1 + lags_at);
+    int32_t *d_lstat = opt_.exact_lag_search ? nullptr : reinterpret_cast<int32_t *>(d_phase1 + status_at);
+    for (size_t i = 0; i < n; ++i) ps[i].stats = reinterpret_cast<double *>(d_phase1) + 10 * i;
+    {
+        size_t v = 0;
+        for (size_t i = 0; i < n; ++i)
+            if (vad_at[i] != SIZE_MAX) vads[v++].loud = reinterpret_cast<uint8_t *>(d_phase1 + loud_at) + vad_at[i];
+    }
+    launch_zero(d_phase1, loud_at, stream_);
     std::vector<LagJob> lag_jobs;
     std::vector<size_t> lag_pair;  // pair of each lag job
-    int32_t *d_lstat = nullptr;    // FP32 form: per lag job, 1 when the f32 search left it undecided
     // aligned energies (read the lags on the device) of the listed pairs
-    auto launch_aligned = [&](const std::vector<size_t> &pairs) {
+    auto plan_aligned = [&](const std::vector<size_t> &pairs) -> Launches {
         std::vector<AlignedEnergyJob> jobs;
         int64_t max_len = 0;
         for (size_t i : pairs) {
@@ -956,12 +1030,15 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
                                             s.stats + 8, s.lag_job ? s.stats + 4 : nullptr});
             max_len = std::max(max_len, (int64_t)s.dl);
         }
-        if (jobs.empty()) return;
+        if (jobs.empty()) return {};
         const int na = (int)jobs.size();
-        if (opt_.form != kFormExact)
-            launch_aligned_energy_tree(upload(jobs), na, arena_.alloc_n<double>((size_t)na * kTreeParts * 3), stream_);
-        else
-            launch_aligned_energy(upload(jobs), na, max_len, arena_.alloc(serial_sum_scratch(na, max_len)), stream_);
+        const AlignedEnergyJob *d = upload(jobs);
+        if (opt_.form != kFormExact) {
+            double *scratch = arena_.alloc_n<double>((size_t)na * kTreeParts * 3);
+            return {[=] { launch_aligned_energy_tree(d, na, scratch, stream_); }};
+        }
+        void *scratch = arena_.alloc(serial_sum_scratch(na, max_len));
+        return {[=] { launch_aligned_energy(d, na, max_len, scratch, stream_); }};
     };
     {
         std::vector<SumJob> sums;
@@ -970,8 +1047,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             if (!s.live) continue;
             const VSig r{s.ref, 0, (int64_t)s.rl, (int64_t)s.rl}, d{s.deg, 0, (int64_t)s.dl, (int64_t)s.dl};
             if (!s.prep) sums.push_back(SumJob{r, s.stats});
-            if (!opt_.disable_global_alignment && s.rl > 0 && s.dl > 0) {
-                s.lag_job = true;
+            if (s.lag_job) {
                 sums.push_back(SumJob{d, s.stats + 4});
                 LagJob j{};
                 j.a = r;
@@ -987,21 +1063,27 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
                 timing_.lag_bytes += lag_search_bytes(j, !opt_.exact_lag_search);
             }
         }
-        launch_sums(sums);
-        record(lag_events_[0]);
-        d_lstat = launch_lag_jobs(lag_jobs, false);
-        record(lag_events_[1]);
         std::vector<size_t> all(n);
         for (size_t i = 0; i < n; ++i) all[i] = i;
-        launch_aligned(all);
+        // every upload of the phase goes up with the first flush
+        const SpecPlan ref_spec = plan_spectrograms(ref_jobs, rc);
+        const Launches do_sums = plan_sums(sums), do_lags = plan_lag_jobs(lag_jobs, false, d_lstat),
+                       do_aligned = plan_aligned(all), do_vad = plan_vad(vads);
+        run_gammatone(ref_spec, side_);
+        VQB_CUDA(cudaEventRecord(ev_ref_done_, side_));
+        run(do_sums);
+        record(lag_events_[0]);
+        run(do_lags);
+        record(lag_events_[1]);
+        run(do_aligned);
+        run(do_vad);
     }
-    int64_t *h_lags = pinned_.alloc_n<int64_t>(n);
-    double *h_stats = pinned_.alloc_n<double>(10 * n);
-    int32_t *h_lstat = d_lstat ? pinned_.alloc_n<int32_t>(lag_jobs.size()) : nullptr;
-    d2h(h_lags, d_lags, n * sizeof(int64_t));
-    for (size_t i = 0; i < n; ++i)
-        if (ps[i].live) d2h(h_stats + 10 * i, ps[i].stats, 10 * sizeof(double));
-    if (h_lstat) d2h(h_lstat, d_lstat, lag_jobs.size() * sizeof(int32_t));
+    char *h_phase1 = static_cast<char *>(pinned_.alloc(phase1_bytes));
+    const int64_t *h_lags = reinterpret_cast<int64_t *>(h_phase1 + lags_at);
+    double *h_stats = reinterpret_cast<double *>(h_phase1);
+    const int32_t *h_lstat = d_lstat ? reinterpret_cast<int32_t *>(h_phase1 + status_at) : nullptr;
+    const uint8_t *h_loud = reinterpret_cast<uint8_t *>(h_phase1 + loud_at);
+    d2h(h_phase1, d_phase1, phase1_bytes);
     record(events_[1]);
     sync();
     {
@@ -1011,11 +1093,8 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         if (!redo.empty()) {
             std::vector<size_t> pairs;
             for (size_t k : redo) pairs.push_back(lag_pair[k]);
-            launch_aligned(pairs);
-            for (size_t i : pairs) {
-                d2h(h_lags + i, d_lags + i, sizeof(int64_t));
-                d2h(h_stats + 10 * i, ps[i].stats, 10 * sizeof(double));
-            }
+            run(plan_aligned(pairs));
+            d2h(h_phase1, d_phase1, phase1_bytes);
             sync();
         }
     }
@@ -1036,6 +1115,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     std::vector<size_t> lohi_at;
     std::vector<StatsJob> stat_jobs;
     int max_width = 0;
+    size_t npatches = 0;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
         if (!s.live) continue;
@@ -1058,14 +1138,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             if (s.prep) {
                 s.idx = s.prep->idx;
             } else if (opt_.speech) {
-                std::vector<double> tmp;
-                const double *hr = s.h_ref;
-                if (!hr) {
-                    tmp.resize(s.rl);
-                    VQB_CUDA(cudaMemcpy(tmp.data(), s.ref, s.rl * sizeof(double), cudaMemcpyDeviceToHost));
-                    hr = tmp.data();
-                }
-                s.idx = host::vad_patch_indices(hr, s.rl, s.nf_ref, P, W, 0.25);
+                s.idx = host::vad_patches(h_loud + vad_at[i], s.nf_ref, P, W, kVadOverlap);
             } else {
                 s.idx = host::ref_patch_indices(s.nf_ref, P);
             }
@@ -1075,7 +1148,20 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             s.fail(e.code, e.what());
             continue;
         }
+        npatches += s.search.np;
+    }
+    // What the host reads after the DP lies in one block: per patch its match
+    // statistics, offset and validity.
+    const size_t per = 3 * NB + 1, offs_at = npatches * per * sizeof(double),
+                 valid_at = offs_at + npatches * sizeof(int64_t), match_bytes = valid_at + npatches;
+    char *d_match = static_cast<char *>(arena_.alloc(match_bytes));
+    size_t patch0 = 0;  // the pair's first patch
+    for (size_t i = 0; i < n; ++i) {
+        PairState &s = ps[i];
+        if (!s.live) continue;
         const size_t np = s.search.np;
+        s.patch0 = patch0;
+        patch0 += np;
         s.width = s.nf_deg;
         for (size_t p = 0; p < np; ++p) s.width = std::max(s.width, (size_t)s.search.hi[p] + P);
         max_width = std::max(max_width, (int)s.width);
@@ -1092,9 +1178,9 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         s.sims = arena_.alloc_n<double>(np * s.nf_deg);
         s.dp = arena_.alloc_n<double>(np * s.nf_deg);
         s.bt = arena_.alloc_n<int64_t>(np * s.nf_deg);
-        s.offs = arena_.alloc_n<int64_t>(np);
-        s.valid = arena_.alloc_n<uint8_t>(np);
-        s.mstats = arena_.alloc_n<double>(np * (3 * NB + 1));
+        s.mstats = reinterpret_cast<double *>(d_match) + s.patch0 * per;
+        s.offs = reinterpret_cast<int64_t *>(d_match + offs_at) + s.patch0;
+        s.valid = reinterpret_cast<uint8_t *>(d_match + valid_at) + s.patch0;
         // aligned[i] = deg[i - lead + skip] (applyLag), scaled (scaleToMatchSpl)
         const VSig src{s.deg + s.al.skip, s.al.lead, (int64_t)s.dl - s.al.skip, s.al.len};
         scale_args.resize(scale_args.size() + scale_args_size());
@@ -1134,46 +1220,49 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     }
 
     // ---- 3: spectrograms, prep, NSIM table, DP, match statistics ----------
-    if (nscale) launch_scale(upload_bytes(scale_args.data(), scale_args.size()), nscale, max_al, stream_);
+    // every upload of the phase goes up with the first flush
+    const SpecPlan deg_spec = plan_spectrograms(spec_jobs, rc);
+    const Launches do_prep = plan_prep_jobs(prep_jobs);
+    const void *d_scale = upload_bytes(scale_args.data(), scale_args.size());
+    const PlaneJob *d_planes = upload(plane_jobs);
+    const RefTermsJob *d_terms = upload(term_jobs);
+    const DpJob *d_dp = upload(dp_jobs);
+    const StatsJob *d_stats = upload(stat_jobs);
+    const bool fast_cells = opt_.form != kFormExact;
+    auto upload_tasks = [&](int w) {
+        std::vector<TableTask> tasks;
+        for (const TableTask &row : table_rows)
+            for (int64_t off0 = row.off0; off0 <= row.hi; off0 += w) {
+                TableTask t = row;
+                t.off0 = (int32_t)off0;
+                tasks.push_back(t);
+            }
+        return std::make_pair((const TableTask *)upload(tasks), (int)tasks.size());
+    };
+    const std::vector<int> widths = table_width_candidates((int)P);
+    std::map<int, std::pair<const TableTask *, int>> tasks{{widths[0], upload_tasks(widths[0])}};
+    flush_uploads();
+    if (nscale) launch_scale(d_scale, nscale, max_al, stream_);
     record(events_[2]);
-    run_gammatone(spec_jobs, stream_);
+    run_gammatone(deg_spec, stream_);
     record(events_[3]);
     VQB_CUDA(cudaStreamWaitEvent(stream_, ev_ref_done_, 0));
-    if (!prep_jobs.empty()) launch_prep_jobs(prep_jobs);
+    run(do_prep);
     record(events_[4]);
-    if (!plane_jobs.empty()) launch_plane(upload(plane_jobs), (int)plane_jobs.size(), nbi, max_width, stream_);
-    if (!term_jobs.empty()) launch_ref_terms(upload(term_jobs), (int)term_jobs.size(), nbi, (int)P, stream_);
+    launch_plane(d_planes, (int)plane_jobs.size(), nbi, max_width, stream_);
+    launch_ref_terms(d_terms, (int)term_jobs.size(), nbi, (int)P, stream_);
     if (!table_rows.empty()) {
-        const bool fast_cells = opt_.form != kFormExact;
         auto launch_width = [&](int w) {
-            std::vector<TableTask> tasks;
-            for (const TableTask &row : table_rows)
-                for (int64_t off0 = row.off0; off0 <= row.hi; off0 += w) {
-                    TableTask t = row;
-                    t.off0 = (int32_t)off0;
-                    tasks.push_back(t);
-                }
-            launch_table(upload(tasks), (int)tasks.size(), nbi, (int)P, fast_cells, w, stream_);
+            if (!tasks.count(w)) tasks[w] = upload_tasks(w);
+            flush_uploads();
+            launch_table(tasks[w].first, tasks[w].second, nbi, (int)P, fast_cells, w, stream_);
         };
-        const int w = tuned(kTuneTable, fast_cells ? 1 : 0, nbi, table_width_candidates((int)P), launch_width, stream_);
-        launch_width(w);
+        launch_width(tuned(kTuneTable, fast_cells ? 1 : 0, nbi, widths, launch_width, stream_));
     }
-    if (!dp_jobs.empty()) launch_dp(upload(dp_jobs), (int)dp_jobs.size(), stream_);
-    if (!stat_jobs.empty()) launch_stats(upload(stat_jobs), (int)stat_jobs.size(), nbi, stream_);
-    std::vector<int64_t *> h_offs(n, nullptr);
-    std::vector<uint8_t *> h_valid(n, nullptr);
-    std::vector<double *> h_ms(n, nullptr);
-    for (size_t i = 0; i < n; ++i) {
-        PairState &s = ps[i];
-        if (!s.live) continue;
-        const size_t np = s.search.np;
-        h_offs[i] = pinned_.alloc_n<int64_t>(np);
-        h_valid[i] = pinned_.alloc_n<uint8_t>(np);
-        h_ms[i] = pinned_.alloc_n<double>(np * (3 * NB + 1));
-        d2h(h_offs[i], s.offs, np * sizeof(int64_t));
-        d2h(h_valid[i], s.valid, np);
-        d2h(h_ms[i], s.mstats, np * (3 * NB + 1) * sizeof(double));
-    }
+    launch_dp(d_dp, (int)dp_jobs.size(), stream_);
+    launch_stats(d_stats, (int)stat_jobs.size(), nbi, stream_);
+    char *h_match = static_cast<char *>(pinned_.alloc(match_bytes));
+    d2h(h_match, d_match, match_bytes);
     record(events_[5]);
     sync();
 
@@ -1190,14 +1279,14 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         s.matches.resize(np);
         for (size_t p = 0; p < np; ++p) {
             host::Match &m = s.matches[p];
-            const double *ms = h_ms[i] + p * (3 * NB + 1);
+            const double *ms = reinterpret_cast<const double *>(h_match) + (s.patch0 + p) * per;
             m.means.assign(ms, ms + NB);
             m.stddevs.assign(ms + NB, ms + 2 * NB);
             m.energy.assign(ms + 2 * NB, ms + 3 * NB);
             m.similarity = ms[3 * NB];
-            const int64_t off = h_offs[i][p];
+            const int64_t off = reinterpret_cast<const int64_t *>(h_match + offs_at)[s.patch0 + p];
             if (off >= 0) {
-                m.valid = h_valid[i][p] != 0;
+                m.valid = h_match[valid_at + s.patch0 + p] != 0;
                 if (m.valid) {
                     m.deg_start = (double)off * fd;
                     m.deg_end = m.deg_start + patch_dur;
@@ -1229,7 +1318,11 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         }
     }
     if (n_slices) {
-        d_slice_lags = arena_.alloc_n<int64_t>(n_slices);
+        // lags and status words in one block
+        const size_t slice_bytes = n_slices * (sizeof(int64_t) + sizeof(int32_t));
+        d_slice_lags = static_cast<int64_t *>(arena_.alloc(slice_bytes));
+        int32_t *d_sstat = opt_.exact_lag_search ? nullptr : reinterpret_cast<int32_t *>(d_slice_lags + n_slices);
+        launch_zero(d_slice_lags, slice_bytes, stream_);
         double *d_sst = arena_.alloc_n<double>(8 * n_slices);
         size_t k = 0;
         for (auto &s : ps) {
@@ -1254,15 +1347,17 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             }
         }
         // ---- 5: slice lags --------------------------------------------------
-        launch_sums(slice_sums);
-        int32_t *d_sstat = launch_lag_jobs(slice_lags, false);
-        int64_t *h_sl = pinned_.alloc_n<int64_t>(n_slices);
-        int32_t *h_sstat = d_sstat ? pinned_.alloc_n<int32_t>(n_slices) : nullptr;
-        d2h(h_sl, d_slice_lags, n_slices * sizeof(int64_t));
-        if (h_sstat) d2h(h_sstat, d_sstat, n_slices * sizeof(int32_t));
+        {
+            const Launches do_sums = plan_sums(slice_sums), do_lags = plan_lag_jobs(slice_lags, false, d_sstat);
+            run(do_sums);
+            run(do_lags);
+        }
+        int64_t *h_sl = static_cast<int64_t *>(pinned_.alloc(slice_bytes));
+        const int32_t *h_sstat = d_sstat ? reinterpret_cast<int32_t *>(h_sl + n_slices) : nullptr;
+        d2h(h_sl, d_slice_lags, slice_bytes);
         sync();
         if (!rerun_undecided(slice_lags, h_sstat, false).empty()) {
-            d2h(h_sl, d_slice_lags, n_slices * sizeof(int64_t));
+            d2h(h_sl, d_slice_lags, slice_bytes);
             sync();
         }
 
@@ -1273,6 +1368,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         std::vector<StatsJob> rstats;
         int max_cols = 0;
         k = 0;
+        double *d_rst = arena_.alloc_n<double>(n_slices * per);  // the slices' statistics, read back together
         for (auto &s : ps) {
             if (!s.live) continue;
             for (auto &rp : s.rps) {
@@ -1287,7 +1383,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
                 rp.ds_raw = arena_.alloc_n<double>(NB * rp.nf);
                 rp.rs = arena_.alloc_n<double>(NB * rp.nf);
                 rp.ds = arena_.alloc_n<double>(NB * rp.nf);
-                rp.st = arena_.alloc_n<double>(3 * NB + 1);
+                rp.st = d_rst + rstats.size() * per;
                 const int64_t g_ref = host::reuse_frame(rp.rl, rp.trim.ref_off, H, rp.nf, s.nf_ref);
                 if (g_ref >= 0) {
                     copies.push_back(CopyJob{s.ref_raw, (int32_t)s.nf_ref, (int32_t)g_ref, rp.rs_raw, (int32_t)rp.nf});
@@ -1315,20 +1411,17 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             }
         }
         // ---- 7: realigned spectrograms and statistics ------------------------
-        if (!copies.empty()) launch_copy_frames(upload(copies), (int)copies.size(), nbi, max_cols, stream_);
-        run_gammatone(rjobs, stream_);
-        if (!rprep.empty()) launch_prep_jobs(rprep);
-        if (!rstats.empty()) launch_stats(upload(rstats), (int)rstats.size(), nbi, stream_);
-        std::vector<double *> h_rst;
-        for (auto &s : ps) {
-            if (!s.live) continue;
-            for (auto &rp : s.rps) {
-                if (rp.nf == 0) continue;
-                double *h = pinned_.alloc_n<double>(3 * NB + 1);
-                d2h(h, rp.st, (3 * NB + 1) * sizeof(double));
-                h_rst.push_back(h);
-            }
-        }
+        const CopyJob *d_copies = upload(copies);
+        const SpecPlan slice_spec = plan_spectrograms(rjobs, rc);
+        const Launches do_rprep = plan_prep_jobs(rprep);
+        const StatsJob *d_rstats = upload(rstats);
+        flush_uploads();
+        launch_copy_frames(d_copies, (int)copies.size(), nbi, max_cols, stream_);
+        run_gammatone(slice_spec, stream_);
+        run(do_rprep);
+        launch_stats(d_rstats, (int)rstats.size(), nbi, stream_);
+        double *h_rst = pinned_.alloc_n<double>(rstats.size() * per);
+        d2h(h_rst, d_rst, rstats.size() * per * sizeof(double));
         record(events_[6]);
         sync();
 
@@ -1338,7 +1431,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             if (!s.live) continue;
             for (auto &rp : s.rps) {
                 if (rp.nf == 0) continue;
-                const double *st = h_rst[q++];
+                const double *st = h_rst + q++ * per;
                 host::Match &m = s.matches[rp.mi];
                 const double sim = st[3 * NB];
                 if (!(sim < m.similarity)) {
@@ -1521,7 +1614,7 @@ void Engine::measure_batch_streamed(size_t n, const double *const *refs, const s
         VQB_CUDA(cudaStreamWaitEvent(stream_, ev_up_[k & 1], 0));
         const size_t b0 = bounds[k], m = bounds[k + 1] - b0;
         measure_batch(m, d_ref.data() + b0, ref_lens + b0, d_deg.data() + b0, deg_lens + b0, sample_rate, true,
-                      part, prepared ? prepared + b0 : nullptr, refs + b0);
+                      part, prepared ? prepared + b0 : nullptr);
         if (next.valid()) next.get();
         for (size_t j = 0; j < m; ++j) out[b0 + j] = std::move(part[j]);
         const Timing &t = timing_;
@@ -1679,6 +1772,7 @@ void Engine::gradients(detail::PairState *ps, size_t n, const size_t *deg_lens, 
         const GradSpecJob *d_jobs = upload(jobs);
         const void *d_tiles = upload_bytes(tiles.data(), tiles.size());
         double *scratch = arena_.alloc_n<double>(gammatone_bwd_scratch_count(ntiles, (int)W));
+        flush_uploads();
         launch_gammatone_bwd(d_jobs, d_tiles, ntiles, rc.d_fast_coeffs, (int)NB, rc.d_hann, (int)W, (int)H, scratch,
                              stream_);
     }

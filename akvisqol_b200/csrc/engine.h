@@ -140,14 +140,12 @@ public:
     // device_inputs. Per-pair failures land in out[i].code.
     // With prepared non-NULL, pair i whose prepared[i] is set takes its
     // reference from there (refs[i] and ref_lens[i] are ignored).
-    // host_refs (device inputs only, may be NULL): host copies of the
-    // references, read by the speech-mode VAD instead of a read-back.
     // grads: also d moslqo / d degraded signal of each pair scored
     // (PairOutcome::grad), the forward's discrete decisions fixed.
     void measure_batch(size_t n, const double *const *refs, const size_t *ref_lens, const double *const *degs,
                        const size_t *deg_lens, uint32_t sample_rate, bool device_inputs,
                        std::vector<PairOutcome> &out, const PreparedRef *const *prepared = nullptr,
-                       const double *const *host_refs = nullptr, bool grads = false);
+                       bool grads = false);
     // Host inputs scored in consecutive chunks of growing size: chunk k+1's
     // signals are copied to the device on a copy stream (from a helper
     // thread, so pageable sources do not block scoring) while chunk k is
@@ -204,9 +202,15 @@ private:
         FastBandCoeffs *d_fast_coeffs = nullptr;
         double *d_hann = nullptr;
     };
-    // Envelope statistics of sum jobs: serial (exact) or tree (fast).
-    void launch_sums(const std::vector<SumJob> &sums);
-    void launch_serial_sums(const std::vector<SumJob> &sums);
+    // A phase's work is planned first (device buffers, job arrays through
+    // upload) and launched after, so that its uploads go up in one copy: run
+    // flushes them, then launches.
+    using Launches = std::vector<std::function<void()>>;
+    void run(const Launches &launches);
+    // Envelope statistics of sum jobs: serial (exact form, or serial) or tree.
+    Launches plan_sums(const std::vector<SumJob> &sums, bool serial = false);
+    VadJob vad_job(const VSig &sig, size_t nf, size_t window, size_t *at) const;
+    Launches plan_vad(const std::vector<VadJob> &jobs);
     // The launch shape for a kernel class among candidates: measured on the
     // caller's jobs at first use per device (launch(c) launches them with
     // shape c on st), then reused; candidates[0] when autotuning is off.
@@ -221,10 +225,19 @@ private:
     // the candidates).
     int tuned(int kernel, int a, int b, const std::vector<int> &candidates, const std::function<void(int)> &launch,
               cudaStream_t st, const std::vector<int> *allowed = nullptr);
-    // Gammatone spectrograms of the jobs in this engine's form on stream st;
-    // returns the RMS count.
-    uint64_t launch_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, cudaStream_t st,
-                                 cudaEvent_t begin = nullptr, cudaEvent_t end = nullptr);
+    // Gammatone spectrograms of the jobs in this engine's form, on stream st.
+    struct SpecPlan {
+        std::vector<SpecJob> jobs;
+        const SpecJob *d_jobs = nullptr;
+        const void *d_tiles = nullptr;
+        int ntiles = 0, frames = 0;  // tiles of `frames` frames
+        uint64_t rms = 0;
+        const RateCache *rc = nullptr;
+    };
+    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc);
+    void run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin = nullptr,
+                          cudaEvent_t end = nullptr);
+    const void *upload_tiles(const std::vector<SpecJob> &jobs, int F, int *ntiles);
     const RateCache &rate_cache(uint32_t sample_rate);
     // d moslqo / d degraded signal of the pairs measure_batch just scored
     // (grad_ok), into out[i].grad: the host reverses of the MOS mapping,
@@ -234,18 +247,19 @@ private:
                    std::vector<PairOutcome> &out);
 
     // Envelope (or raw) lag search for jobs whose a/b/stat pointers are set;
-    // lags land in the jobs' lag_out (device). Launches only. The FP32 form
-    // (unless `exact`) runs the f32 search and returns a device array of one
-    // status word per job, in job order: 1 where the f32 search left the job
-    // undecided (its lag_out is untouched); the caller reads it back with the
-    // lags and passes it to rerun_undecided. Else returns null.
-    int32_t *launch_lag_jobs(std::vector<LagJob> &jobs, bool raw, bool exact = false);
+    // lags land in the jobs' lag_out (device). With d_status (one zeroed word
+    // per job) the f32 search runs, and sets it to 1 where it left the job
+    // undecided (its lag_out is untouched): the caller reads it back with the
+    // lags and passes it to rerun_undecided. Without, the exact search.
+    Launches plan_lag_jobs(const std::vector<LagJob> &jobs, bool raw, int32_t *d_status);
     // The jobs whose status (host copy) is 1, rerun with the exact search;
     // returns their indices (launches only; nothing when none).
     std::vector<size_t> rerun_undecided(const std::vector<LagJob> &jobs, const int32_t *h_status, bool raw);
     template <class T>
     T *upload(const std::vector<T> &v);
     void *upload_bytes(const void *src, size_t bytes);
+    void flush_uploads();
+    void begin_batch();
     void d2h(void *dst, const void *src, size_t bytes);
     void sync();
     void record(cudaEvent_t e);
@@ -260,6 +274,9 @@ private:
     cudaStream_t stream_ = nullptr;
     Arena arena_;
     PinnedArena pinned_;
+    // the chunk small uploads gather in, and its range not yet sent
+    char *up_host_ = nullptr, *up_dev_ = nullptr;
+    size_t up_cap_ = 0, up_begin_ = 0, up_end_ = 0;
     std::map<uint32_t, RateCache> rates_;
     std::map<size_t, Twiddles> twiddles_;
     std::vector<cudaEvent_t> events_;

@@ -223,30 +223,19 @@ std::vector<int64_t> ref_patch_indices(size_t nf, size_t patch) {
     return idx;
 }
 
-std::vector<int64_t> vad_patch_indices(const double *ref, size_t len, size_t nf, size_t patch, size_t window,
-                                       double overlap) {
+size_t vad_chunks(size_t nf, size_t patch, size_t window, double overlap) {
     const double frame_size = (double)window * overlap;
     const size_t frame_len = (size_t)frame_size;
-    const size_t patch_len = (size_t)((double)patch * frame_size);
     const size_t first = patch / 2 - 1;
+    if (nf <= first || frame_len == 0) return 0;
+    return (nf - first) / patch * (size_t)((double)patch * frame_size) / frame_len;
+}
+
+std::vector<int64_t> vad_patches(const uint8_t *loud, size_t nf, size_t patch, size_t window, double overlap) {
+    const size_t first = patch / 2 - 1, frame_len = (size_t)((double)window * overlap);
     std::vector<int64_t> out;
     if (nf <= first || frame_len == 0) return out;
-    const size_t patches = (nf - first) / patch;
-    const size_t chunks = patches * patch_len / frame_len;
-    double peak = -kInf;
-    for (size_t i = 0; i < len; ++i) peak = std::fmax(peak, ref[i]);
-    // RMS of int16-scaled chunks, starting at *sample* `first` (upstream quirk).
-    std::vector<char> loud(chunks);
-    for (size_t c = 0; c < chunks; ++c) {
-        double sq = 0.0;
-        for (size_t j = 0; j < frame_len; ++j) {
-            const size_t k = first + c * frame_len + j;
-            const double x = k < len ? ref[k] / peak : 0.0;
-            const double s = std::trunc(std::min(std::max(x * 32768.0, -32768.0), 32767.0));
-            sq += s * s;
-        }
-        loud[c] = std::sqrt(sq / (double)frame_len) >= 5000.0;
-    }
+    const size_t patches = (nf - first) / patch, chunks = vad_chunks(nf, patch, window, overlap);
     // A chunk is silent only when it and the two before it are quiet; the
     // first two always count as active.
     std::vector<double> vad(std::max<size_t>(chunks, 2), 0.0);
@@ -260,6 +249,27 @@ std::vector<int64_t> vad_patch_indices(const double *ref, size_t len, size_t nf,
         if (act >= 1.0) out.push_back((int64_t)start);
     }
     return out;
+}
+
+std::vector<int64_t> vad_patch_indices(const double *ref, size_t len, size_t nf, size_t patch, size_t window,
+                                       double overlap) {
+    const size_t frame_len = (size_t)((double)window * overlap);
+    const size_t first = patch / 2 - 1, chunks = vad_chunks(nf, patch, window, overlap);
+    double peak = -kInf;
+    for (size_t i = 0; i < len; ++i) peak = std::fmax(peak, ref[i]);
+    // RMS of int16-scaled chunks, starting at *sample* `first` (upstream quirk).
+    std::vector<uint8_t> loud(chunks);
+    for (size_t c = 0; c < chunks; ++c) {
+        double sq = 0.0;
+        for (size_t j = 0; j < frame_len; ++j) {
+            const size_t k = first + c * frame_len + j;
+            const double x = k < len ? ref[k] / peak : 0.0;
+            const double s = std::trunc(std::min(std::max(x * 32768.0, -32768.0), 32767.0));
+            sq += s * s;
+        }
+        loud[c] = std::sqrt(sq / (double)frame_len) >= 5000.0;
+    }
+    return vad_patches(loud.data(), nf, patch, window, overlap);
 }
 
 size_t max_num_patches(const std::vector<int64_t> &idx, size_t nf_deg, size_t patch) {

@@ -64,6 +64,11 @@ std::vector<int64_t> ref_patch_indices(size_t nf, size_t patch);
 // vad.refPatchIndices (reference src/vad.zig:15-81).
 std::vector<int64_t> vad_patch_indices(const double *ref, size_t len, size_t nf, size_t patch, size_t window,
                                        double overlap);
+// The same in two halves: the chunks whose loudness decides (0: no patches),
+// and the patches from those flags (1: the chunk's RMS reaches the VAD's
+// threshold), which the device forms.
+size_t vad_chunks(size_t nf, size_t patch, size_t window, double overlap);
+std::vector<int64_t> vad_patches(const uint8_t *loud, size_t nf, size_t patch, size_t window, double overlap);
 // calcMaxNumPatches (reference src/dp.zig:73-87).
 size_t max_num_patches(const std::vector<int64_t> &idx, size_t nf_deg, size_t patch);
 

@@ -169,6 +169,49 @@ __global__ void __launch_bounds__(256) pack_kernel(const LagJob *__restrict__ jo
     }
 }
 
+// ---- speech VAD -------------------------------------------------------------
+// The samples scale to the signal's peak and truncate to int16, so a chunk's
+// sum of squares is an integer far below 2^53: any order gives the CPU's sum.
+
+// Partial maxima (NaN samples left out, as the CPU's @max).
+__global__ void __launch_bounds__(kTreeThreads) vad_peak_kernel(const VadJob *__restrict__ jobs,
+                                                                double *__restrict__ scratch) {
+    __shared__ double sm[kTreeThreads / 32];
+    const VadJob job = jobs[blockIdx.y];
+    int64_t lo, hi;
+    part_range(job.sig.len, lo, hi);
+    double m = -INFINITY;
+#pragma unroll 4
+    for (int64_t k = lo + threadIdx.x; k < hi; k += kTreeThreads) m = fmax(m, vsig_at(job.sig, k));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kTreeThreads / 32; ++w) m = fmax(m, sm[w]);
+        scratch[(int64_t)blockIdx.y * kTreeParts + blockIdx.x] = m;
+    }
+}
+
+// A warp per chunk.
+__global__ void __launch_bounds__(128) vad_loud_kernel(const VadJob *__restrict__ jobs,
+                                                       const double *__restrict__ scratch) {
+    const VadJob job = jobs[blockIdx.y];
+    const int lane = threadIdx.x & 31, c = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (c >= job.chunks) return;
+    double peak = scratch[(int64_t)blockIdx.y * kTreeParts + lane];
+    for (int o = 16; o > 0; o >>= 1) peak = fmax(peak, __shfl_xor_sync(0xffffffffu, peak, o));
+    const int64_t k0 = job.first + (int64_t)c * job.frame_len;
+    double sq = 0.0;
+    for (int j = lane; j < job.frame_len; j += 32) {
+        const int64_t k = k0 + j;
+        const double v = (k < job.sig.len ? vsig_at(job.sig, k) / peak : 0.0) * 32768.0;
+        const double s = trunc(v < -32768.0 ? -32768.0 : v > 32767.0 ? 32767.0 : v);  // (NaN stays)
+        sq += s * s;
+    }
+    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    if (lane == 0) job.loud[c] = sqrt(sq / (double)job.frame_len) >= 5000.0 ? 1 : 0;
+}
+
 // out[i] = aligned(i) * factor: scaleToMatchSpl on the lag-aligned signal
 // (reference src/audio.zig:152-158; x * 1.0 == x when unscaled).
 struct ScaleArgs {
@@ -204,6 +247,13 @@ void launch_aligned_energy_tree(const AlignedEnergyJob *a, int njobs, double *d_
     if (njobs <= 0) return;
     aligned_tree_parts<<<dim3(kTreeParts, (unsigned)njobs), kTreeThreads, 0, s>>>(a, d_scratch);
     aligned_tree_finish<<<njobs, 32, 0, s>>>(a, d_scratch);
+    launch_counter() += 2;
+}
+
+void launch_vad(const VadJob *d_jobs, int njobs, int max_chunks, double *d_scratch, cudaStream_t s) {
+    if (njobs <= 0 || max_chunks <= 0) return;
+    vad_peak_kernel<<<dim3(kTreeParts, (unsigned)njobs), kTreeThreads, 0, s>>>(d_jobs, d_scratch);
+    vad_loud_kernel<<<dim3((unsigned)((max_chunks + 3) / 4), (unsigned)njobs), 128, 0, s>>>(d_jobs, d_scratch);
     launch_counter() += 2;
 }
 

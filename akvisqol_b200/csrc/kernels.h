@@ -92,6 +92,10 @@ size_t scale_args_size();
 void fill_scale_args(void *dst, const VSig &src, double factor, double *out);
 void launch_scale(const void *d_args, int njobs, int64_t max_len, cudaStream_t s);
 
+// Chunk loudness of the jobs' references (speech mode's VAD); max_chunks: the
+// most chunks of a job; scratch: kTreeParts doubles per job.
+void launch_vad(const VadJob *d_jobs, int njobs, int max_chunks, double *d_scratch, cudaStream_t s);
+
 // Fast form: the same statistics as deterministic tree reductions.
 // scratch: kTreeParts * 3 doubles per job.
 constexpr int kTreeParts = 32;

@@ -223,3 +223,30 @@ def test_fast_quotient_within_one_ulp(native):
     assert np.all(np.isfinite(got))
     assert float(err.max()) <= 1.0, float(err.max())
     assert float(np.mean(got == want)) > 0.99
+
+
+@pytest.mark.parametrize("seconds", [0.61, 1.0, 2.37, 4.0])
+@pytest.mark.parametrize("kind", ["speech", "quiet", "negative", "spikes"])
+def test_vad_patches(native, oracle, kind, seconds):
+    """The VAD's patches (chunk loudness formed on the device) against the
+    oracle's: signals that end inside a chunk, that stay near the loudness
+    threshold, that never rise above zero, and whose peak is one sample."""
+    from akvisqol_b200 import synth
+    ref, deg = synth.speech_pair(synth.SEED_BASE + 77, seconds=seconds)
+    rng = np.random.default_rng(int(seconds * 100))
+    if kind == "quiet":
+        ref = 0.3 * rng.uniform(-1.0, 1.0, ref.size) * (0.3 + 0.7 * (np.arange(ref.size) // 900 % 2))
+    elif kind == "negative":
+        ref = -np.abs(ref) - 1e-3
+    elif kind == "spikes":
+        ref = 0.1 * ref
+        ref[ref.size // 2] = 1.0
+    window, hop = oracle.window_hop(16000)
+    nf = 1 + (ref.size - window) // hop
+    want = oracle.vad_patch_indices(ref, nf, 20, window)
+    ctx = native.Context(mode=native.MODE_SPEECH, use_lattice_model=False, precision="balanced")
+    (code, _, tr), = ctx.measure_batch_traced([ref], [ref], 16000)
+    if len(want) == 0:
+        assert code == native.E_SIGNAL
+    else:
+        assert code == 0 and list(tr["ref_index"]) == list(want)[:tr["num_patches"]] and tr["num_patches"] >= len(want) - 1
