@@ -163,6 +163,7 @@ Engine::Engine(int device, const Options &opt, std::shared_ptr<const host::Svr> 
     lag_init_attributes();
     lag32_init_attributes();
     nsim_init_attributes();
+    spectral_init_attributes();
     VQB_CUDA(cudaGetLastError());
 }
 
@@ -183,6 +184,7 @@ Engine::~Engine() {
         cudaFree(kv.second.d_coeffs);
         cudaFree(kv.second.d_fast_coeffs);
         cudaFree(kv.second.d_hann);
+        cudaFree(kv.second.d_spectral);
     }
     for (auto &kv : twiddles_) cudaFree(const_cast<double2 *>(kv.second.top));
     for (auto e : events_) cudaEventDestroy(e);
@@ -219,13 +221,40 @@ const Engine::RateCache &Engine::rate_cache(uint32_t sr) {
     // plain cudaMemcpy may return before its DMA lands, and the engine's
     // non-blocking streams would not wait for it).
     std::vector<FastBandCoeffs> fast(nb_);
-    fill_fast_band_coeffs(rc.fb.run.data(), rc.fb.cf.data(), (int)nb_, fast.data());
+    fill_fast_band_coeffs(rc.fb.run.data(), (int)nb_, fast.data());
     VQB_CUDA(cudaMalloc(&rc.d_fast_coeffs, nb_ * sizeof(FastBandCoeffs)));
     VQB_CUDA(cudaMemcpyAsync(rc.d_coeffs, rc.fb.run.data(), nb_ * sizeof(BandCoeffs), cudaMemcpyHostToDevice, stream_));
     VQB_CUDA(cudaMemcpyAsync(rc.d_fast_coeffs, fast.data(), nb_ * sizeof(FastBandCoeffs), cudaMemcpyHostToDevice,
                              stream_));
     if (!w.empty())
         VQB_CUDA(cudaMemcpyAsync(rc.d_hann, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, stream_));
+    if (opt_.form != kFormExact && spectral_window(rc.geo.window)) {
+        rc.spectral = spectral_tables(rc.fb.run, rc.geo.window);
+        const SpectralTables &t = *rc.spectral;
+        // one allocation, each table at a 256-byte boundary
+        size_t bytes = 0;
+        std::vector<std::pair<const void *, size_t>> parts;
+        std::vector<size_t> at;
+        auto add = [&](const auto &v) {
+            parts.emplace_back(v.data(), v.size() * sizeof(v[0]));
+            at.push_back(bytes);
+            bytes += (parts.back().second + 255) / 256 * 256;
+        };
+        add(t.hann), add(t.weights), add(t.tails), add(t.twiddles), add(t.wide), add(t.narrow), add(t.quad_slot),
+            add(t.quad_segs);
+        VQB_CUDA(cudaMalloc(&rc.d_spectral, bytes));
+        char *d = static_cast<char *>(rc.d_spectral);
+        for (size_t i = 0; i < parts.size(); ++i)
+            VQB_CUDA(cudaMemcpyAsync(d + at[i], parts[i].first, parts[i].second, cudaMemcpyHostToDevice, stream_));
+        rc.spectral_dev.hann = reinterpret_cast<const double *>(d + at[0]);
+        rc.spectral_dev.weights = reinterpret_cast<const double *>(d + at[1]);
+        rc.spectral_dev.tails = reinterpret_cast<const double *>(d + at[2]);
+        rc.spectral_dev.twiddles = reinterpret_cast<const double2 *>(d + at[3]);
+        rc.spectral_dev.wide = reinterpret_cast<const SpectralTask *>(d + at[4]);
+        rc.spectral_dev.narrow = reinterpret_cast<const SpectralTask *>(d + at[5]);
+        rc.spectral_dev.quad_slot = reinterpret_cast<const int32_t *>(d + at[6]);
+        rc.spectral_dev.quad_segs = reinterpret_cast<const int32_t *>(d + at[7]);
+    }
     VQB_CUDA(cudaStreamSynchronize(stream_));
     return rates_.emplace(sr, std::move(rc)).first->second;
 }
@@ -457,10 +486,15 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
     const size_t np = nfr / std::max<size_t>(1, P) + 1;
     const size_t n_global = host::fft_size_for(std::max(rl, dl));
     const size_t n_slice = host::fft_size_for(2 * P * H + 2);
+    // FMA forms: a frame's spectrum and partial sums (k_spectral.cu), launches of
+    // at most 2048 frames; the degraded and realigned spectrograms share theirs
+    auto spectral_frames = [](size_t nf) { return std::min<size_t>(nf + 63, 2048); };
+    const size_t spectral = 5 * host::fft_size_for(host::analysis_geometry(sample_rate).window) *
+                            (spectral_frames(nfr) + spectral_frames(std::max(nfd, 2 * np * (P + 2))));
     const size_t sums = 2 * serial_sum_scratch(2, (int64_t)std::max(rl, dl)) +
                         serial_sum_scratch((int)(2 * np), (int64_t)(2 * P * H + 2));
     size_t b = 8 * (rl + dl)                                   // inputs
-               + sums                                          // the exact form's serial sums
+               + std::max(sums, spectral)                      // exact form's sums, FMA forms' spectra
                + 16 * n_global + 16 * 1024                     // lag search and argmax parts
                + 8 * al                                        // aligned, scaled degraded signal
                + 8 * NB * (2 * nfr + 2 * nfd + 4 * width)      // spectrograms, prepared copies, plane
@@ -483,79 +517,62 @@ const void *Engine::upload_tiles(const std::vector<SpecJob> &jobs, int F, int *n
     return upload_bytes(tiles.data(), tiles.size());
 }
 
-Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc) {
+Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc,
+                                           const SpecPlan *before) {
     SpecPlan plan;
-    plan.jobs = jobs;
-    plan.d_jobs = upload(jobs);
-    for (const SpecJob &j : jobs) plan.rms += (uint64_t)j.nf * nb_;
+    plan.rc = &rc;
+    for (const SpecJob &j : jobs) plan.frames += (size_t)j.nf;
+    plan.rms = (uint64_t)plan.frames * nb_;
+    if (jobs.empty()) return plan;
     const int nbi = (int)nb_;
+    if (rc.spectral) {
+        // a descriptor per frame: where its samples lie, which of them the
+        // signal holds, where its RMS values go
+        const int64_t W = (int64_t)rc.geo.window, H = (int64_t)rc.geo.hop;
+        std::vector<SpectralFrame> frames((size_t)spectral_frame_count((int)plan.frames), SpectralFrame{});
+        size_t k = 0;
+        for (const SpecJob &j : jobs)
+            for (int64_t f = 0; f < j.nf; ++f) {
+                const int64_t first = f * H - j.sig.head;  // base index of sample 0
+                const int64_t lo = std::min(W, std::max<int64_t>(0, -first));
+                const int64_t hi = std::max(lo, std::min(W, j.sig.avail - first));
+                frames[k++] = SpectralFrame{j.sig.base + first, j.out + f, (int32_t)lo, (int32_t)hi, j.nf};
+            }
+        plan.d_frames = upload(frames);
+        plan.scratch_count = spectral_scratch_count(*rc.spectral, (int)plan.frames);
+        plan.scratch = before && before->scratch_count >= plan.scratch_count
+                           ? before->scratch
+                           : arena_.alloc_n<double>(plan.scratch_count);
+        return plan;
+    }
     if (opt_.form == kFormExact) {
         // a rule's shape (VISQOL_TUNE_0 may fix another)
         const std::vector<int> shapes = gammatone_frames_shapes(nbi);
-        plan.frames = tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, [](int) {}, stream_, &shapes);
+        plan.tile = tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, [](int) {}, stream_, &shapes);
     } else {
-        plan.frames = gammatone_fast_frames_per_cta();
+        plan.tile = gammatone_staged_frames_per_cta();
     }
-    plan.d_tiles = upload_tiles(jobs, plan.frames, &plan.ntiles);
-    plan.rc = &rc;
+    plan.d_jobs = upload(jobs);
+    plan.d_tiles = upload_tiles(jobs, plan.tile, &plan.ntiles);
     return plan;
 }
 
 void Engine::run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin, cudaEvent_t end) {
-    if (plan.jobs.empty()) return;
+    if (!plan.frames) return;
     const RateCache &rc = *plan.rc;
-    const SpecJob *d_jobs = plan.d_jobs;
-    const int nbi = (int)nb_;
-    const int W = (int)rc.geo.window, H = (int)rc.geo.hop;
-    // uploads go up on the main stream; a side stream waits for them
-    auto uploaded = [&] {
-        flush_uploads();
-        if (st != stream_) {
-            record(ev_inputs_);
-            VQB_CUDA(cudaStreamWaitEvent(st, ev_inputs_, 0));
-        }
-    };
-    uploaded();
-    if (opt_.form == kFormF32) {
-        int *queue = arena_.alloc_n<int>(1);  // the persistent form's work counter
-        auto launch = [&](int shape) {
-            if (shape >= 100) launch_zero(queue, sizeof(int), st);
-            launch_gammatone_fast(d_jobs, plan.d_tiles, plan.ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, shape, queue,
-                                  st);
-        };
-        static const std::vector<int> all_shapes = gammatone_fast_shapes();
-        const int shape =
-            tuned(kTuneGammatoneFastCtas, opt_.form, nbi, gammatone_fast_shape_candidates(), launch, st, &all_shapes);
-        if (begin) VQB_CUDA(cudaEventRecord(begin, st));
-        launch(shape);
-    } else if (opt_.form == kFormF64) {
-        // the FP64-FMA kernel at its measured shape, or the same form on the
-        // FP32 kernel's staged tiles (same bits); tile lists on first use
-        std::map<int, std::pair<const void *, int>> lists;
-        auto launch_frames = [&](int F) {
-            auto &l = lists[F];
-            if (!l.first) {
-                l.first = upload_tiles(plan.jobs, F, &l.second);
-                uploaded();
-            }
-            launch_gammatone_f64fma(d_jobs, l.first, l.second, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, F, st);
-        };
-        const int F = tuned(kTuneGammatone, opt_.form, nbi, gammatone_f64fma_frames_candidates(nbi), launch_frames, st);
-        auto launch = [&](int staged) {
-            if (staged)
-                launch_gammatone_f64_staged(d_jobs, plan.d_tiles, plan.ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H,
-                                            st);
-            else
-                launch_frames(F);
-        };
-        const int staged =
-            tuned(kTuneGammatoneF64Staged, opt_.form, nbi, gammatone_f64_staged_candidates(), launch, st);
-        if (begin) VQB_CUDA(cudaEventRecord(begin, st));
-        launch(staged);
-    } else {
-        if (begin) VQB_CUDA(cudaEventRecord(begin, st));
-        launch_gammatone(d_jobs, plan.d_tiles, plan.ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, plan.frames, st);
+    const int nbi = (int)nb_, W = (int)rc.geo.window, H = (int)rc.geo.hop;
+    flush_uploads();
+    if (st != stream_) {  // uploads go up on the main stream
+        record(ev_inputs_);
+        VQB_CUDA(cudaStreamWaitEvent(st, ev_inputs_, 0));
     }
+    if (begin) VQB_CUDA(cudaEventRecord(begin, st));
+    if (plan.d_frames)
+        launch_spectral(*rc.spectral, rc.spectral_dev, rc.d_fast_coeffs, plan.d_frames, (int)plan.frames, plan.scratch, st);
+    else if (opt_.form == kFormExact)
+        launch_gammatone(plan.d_jobs, plan.d_tiles, plan.ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, plan.tile, st);
+    else
+        launch_gammatone_staged(plan.d_jobs, plan.d_tiles, plan.ntiles, rc.d_fast_coeffs, nbi, rc.d_hann, W, H, st);
     if (end) VQB_CUDA(cudaEventRecord(end, st));
 }
 
@@ -967,7 +984,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         return {[=] { launch_prep(d, count, nbi, max_frames, scratch, stream_); }};
     };
     auto run_gammatone = [&](const SpecPlan &plan, cudaStream_t st) {
-        if (plan.jobs.empty()) return;
+        if (!plan.frames) return;
         const size_t slot = 2 * timing_.gammatone_launches;
         run_spectrograms(plan, st, gt_events_[slot], gt_events_[slot + 1]);
         timing_.gammatone_launches += 1;
@@ -1412,7 +1429,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         }
         // ---- 7: realigned spectrograms and statistics ------------------------
         const CopyJob *d_copies = upload(copies);
-        const SpecPlan slice_spec = plan_spectrograms(rjobs, rc);
+        const SpecPlan slice_spec = plan_spectrograms(rjobs, rc, &deg_spec);
         const Launches do_rprep = plan_prep_jobs(rprep);
         const StatsJob *d_rstats = upload(rstats);
         flush_uploads();

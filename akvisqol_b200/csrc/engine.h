@@ -201,6 +201,10 @@ private:
         BandCoeffs *d_coeffs = nullptr;
         FastBandCoeffs *d_fast_coeffs = nullptr;
         double *d_hann = nullptr;
+        // FMA forms, windows the spectral kernels serve
+        std::shared_ptr<const SpectralTables> spectral;
+        SpectralDevice spectral_dev;
+        void *d_spectral = nullptr;
     };
     // A phase's work is planned first (device buffers, job arrays through
     // upload) and launched after, so that its uploads go up in one copy: run
@@ -217,9 +221,7 @@ private:
     enum TuneKernel {
         kTuneGammatone = 0,
         kTuneTable = 1,
-        kTuneLagColumns = 2,
-        kTuneGammatoneFastCtas = 3,
-        kTuneGammatoneF64Staged = 4
+        kTuneLagColumns = 2
     };
     // VISQOL_TUNE_<kernel> may fix the shape to one of `allowed` (default:
     // the candidates).
@@ -227,14 +229,18 @@ private:
               cudaStream_t st, const std::vector<int> *allowed = nullptr);
     // Gammatone spectrograms of the jobs in this engine's form, on stream st.
     struct SpecPlan {
-        std::vector<SpecJob> jobs;
-        const SpecJob *d_jobs = nullptr;
-        const void *d_tiles = nullptr;
-        int ntiles = 0, frames = 0;  // tiles of `frames` frames
-        uint64_t rms = 0;
         const RateCache *rc = nullptr;
+        size_t frames = 0;
+        uint64_t rms = 0;
+        const SpectralFrame *d_frames = nullptr;  // the spectral kernels' frames, or
+        double *scratch = nullptr;
+        size_t scratch_count = 0;
+        const SpecJob *d_jobs = nullptr;  // the recurrence kernels' jobs and tiles of `tile` frames
+        const void *d_tiles = nullptr;
+        int ntiles = 0, tile = 0;
     };
-    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc);
+    // before: a plan run earlier on the same stream, whose scratch may be used again
+    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, const SpecPlan *before = nullptr);
     void run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin = nullptr,
                           cudaEvent_t end = nullptr);
     const void *upload_tiles(const std::vector<SpecJob> &jobs, int F, int *ntiles);

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "device.cuh"
+#include "spectral_tables.h"
 
 namespace vqb {
 
@@ -48,28 +49,20 @@ struct DpJob {
     uint8_t *valid;   // np
 };
 
-// Per-band coefficients of the fast gammatone forms (k_gammatone_fast.cu).
-// Every stage is a biquad with the band's pole pair and a numerator
+// Per-band coefficients of the FMA forms' cascade (k_gammatone_fast.cu and the
+// gradient). Every stage is a biquad with the band's pole pair and a numerator
 // normalised to 1 + beta z^-1; the numerator gains are one factor, post64.
 struct FastBandCoeffs {
-    double d1, d2;             // poles, all four stages
-    double beta64[4];          // f64 numerators of stages 1-4
-    double post64;             // |s1n0 a0^3|, applied to the RMS
-    float beta[2];             // f32 form: numerators of stages 3-4
-    float p1h, p1l, p2h, p2l;  // f32 form: poles d1, d2 as hi + lo f32 pairs
-    int32_t arith;             // f32 form, per band group: kArith* below
+    double d1, d2;     // poles, all four stages
+    double beta64[4];  // numerators of stages 1-4
+    double post64;     // |s1n0 a0^3|, applied to the RMS
 };
-
-// Arithmetic of a band group in the f32 form's gammatone kernel.
-constexpr int32_t kArithF32Df2t = 0;  // stages 3-4 f32, transposed direct form II
-constexpr int32_t kArithF32Df1 = 1;   // stages 3-4 f32, direct form I
-constexpr int32_t kArithF64 = 2;      // all four stages f64 (poles nearest the unit circle)
 
 // Arithmetic forms of the batch pipeline.
 enum Form : int32_t {
     kFormExact = 0,  // f64, no FMA, the CPU's operation order (bit-identical stages)
-    kFormF32 = 1,    // gammatone stages 3-4 in f32 but in the lowest band group, tree-summed statistics
-    kFormF64 = 2,    // gammatone in f64 with FMA (direct form I), tree-summed statistics
+    kFormF32 = 1,    // as kFormF64 (the form for scores of single precision)
+    kFormF64 = 2,    // gammatone in f64 with FMA (spectral energies), tree-summed statistics
 };
 
 // Kernels launched by this thread so far (each launcher counts its own).
@@ -161,30 +154,34 @@ void launch_gammatone(const SpecJob *d_jobs, const void *d_tiles, int ntiles, co
                       const double *d_hann, int window, int hop, int frames_per_cta, cudaStream_t s);
 void launch_copy_frames(const CopyJob *d_jobs, int njobs, int nb, int max_cols, cudaStream_t s);
 
-// k_gammatone_fast.cu (tiles as fill_gammatone_tile writes them)
-int gammatone_fast_frames_per_cta();
-void fill_fast_band_coeffs(const BandCoeffs *run, const double *cf, int nb, FastBandCoeffs *out);
-// shape: one of gammatone_fast_shape_candidates(): CTAs per SM (register
-// budget), plus 100 for the persistent form, which takes its tiles from a
-// work queue: d_queue, one int that is zero when the launch starts.
-std::vector<int> gammatone_fast_shape_candidates();  // measured by the autotuner
-std::vector<int> gammatone_fast_shapes();            // all valid shapes
-void launch_gammatone_fast(const SpecJob *d_jobs, const void *d_tiles, int ntiles, const FastBandCoeffs *d_coeffs,
-                           int nb, const double *d_hann, int window, int hop, int shape, int *d_queue,
-                           cudaStream_t s);
-// f64 FMA form: two frames per thread; tiles of frames_per_cta frames, one
-// of gammatone_f64fma_frames_candidates(nb) (the first is the default).
-std::vector<int> gammatone_f64fma_frames_candidates(int nb);
-void launch_gammatone_f64fma(const SpecJob *d_jobs, const void *d_tiles, int ntiles, const FastBandCoeffs *d_coeffs,
-                             int nb, const double *d_hann, int window, int hop, int frames_per_cta, cudaStream_t s);
-// The f64 FMA form on the FP32 kernel's staged tiles (tiles of
-// gammatone_fast_frames_per_cta() frames): the same bits as
-// launch_gammatone_f64fma. Candidates of the autotuner: 1 = this one (the
-// default), 0 = that kernel.
-std::vector<int> gammatone_f64_staged_candidates();
-void launch_gammatone_f64_staged(const SpecJob *d_jobs, const void *d_tiles, int ntiles,
-                                 const FastBandCoeffs *d_coeffs, int nb, const double *d_hann, int window, int hop,
-                                 cudaStream_t s);
+// k_spectral.cu: the FMA forms' spectrograms of the windows spectral_window
+// admits, 17 to 32 bands.
+struct SpectralFrame {
+    const double *p;  // sample i of the frame is p[i] for lo <= i < hi, else 0 (i < window)
+    double *out;      // band b's RMS goes to out[b * stride]
+    int32_t lo, hi;
+    int64_t stride;
+};
+struct SpectralDevice {  // SpectralTables on the device
+    const double *hann = nullptr, *weights = nullptr, *tails = nullptr;
+    const double2 *twiddles = nullptr;
+    const SpectralTask *wide = nullptr, *narrow = nullptr;
+    const int32_t *quad_slot = nullptr, *quad_segs = nullptr;
+};
+void spectral_init_attributes();
+// d_frames: spectral_frame_count(nframes) entries, empty ones (lo = hi = 0)
+// behind the last; d_scratch: spectral_scratch_count doubles.
+int spectral_frame_count(int nframes);
+size_t spectral_scratch_count(const SpectralTables &t, int nframes);
+void launch_spectral(const SpectralTables &t, const SpectralDevice &d, const FastBandCoeffs *d_coeffs,
+                     const SpectralFrame *d_frames, int nframes, double *d_scratch, cudaStream_t s);
+
+// k_gammatone_fast.cu: the FMA forms' recurrence (tiles as fill_gammatone_tile
+// writes them, of gammatone_staged_frames_per_cta() frames).
+int gammatone_staged_frames_per_cta();
+void fill_fast_band_coeffs(const BandCoeffs *run, int nb, FastBandCoeffs *out);
+void launch_gammatone_staged(const SpecJob *d_jobs, const void *d_tiles, int ntiles, const FastBandCoeffs *d_coeffs,
+                             int nb, const double *d_hann, int window, int hop, cudaStream_t s);
 
 // k_grad.cu: the gammatone spectrogram's reverse (FP64-FMA arithmetic).
 // Tiles as fill_gammatone_tile writes them, of gammatone_bwd_frames_per_cta()
