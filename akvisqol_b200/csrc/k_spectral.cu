@@ -378,22 +378,57 @@ __global__ void __launch_bounds__(128, 2) energy_kernel(const SpectralFrame *__r
         power_task<NT>(task, weights, power + (int64_t)f0 * row, row, cap, power_part + f0);
 }
 
-// A band's RMS by the recurrence (the operations of k_gammatone_fast.cu), the
-// four stages a sample apart so that a step's four chains are independent.
-__device__ __noinline__ double recurrence(const SpectralFrame &fr, const double *__restrict__ hann, int window,
-                                          const FastBandCoeffs &k) {
-    const double b0 = k.beta64[0], b1 = k.beta64[1], b2 = k.beta64[2], b3 = k.beta64[3], nd1 = -k.d1, nd2 = -k.d2;
-    double xp = 0.0, a1 = 0.0, a2 = 0.0, e1 = 0.0, e2 = 0.0, g1 = 0.0, g2 = 0.0, y1 = 0.0, y2 = 0.0, acc = 0.0;
-    for (int i = 0; i < window + 3; ++i) {
-        const double x = i < window && i >= fr.lo && i < fr.hi ? fr.p[i] * hann[i] : 0.0;
-        const double y = __fma_rn(nd1, y1, __fma_rn(nd2, y2, __fma_rn(b3, g2, g1)));
-        const double g = __fma_rn(nd1, g1, __fma_rn(nd2, g2, __fma_rn(b2, e2, e1)));
-        const double e = __fma_rn(nd1, e1, __fma_rn(nd2, e2, __fma_rn(b1, a2, a1)));
-        const double a = __fma_rn(nd1, a1, __fma_rn(nd2, a2, __fma_rn(b0, xp, x)));
-        y2 = y1, y1 = y, g2 = g1, g1 = g, e2 = e1, e1 = e, a2 = a1, a1 = a, xp = x;
-        acc = __fma_rn(y, y, acc);
+// A band's RMS by the recurrence (the operations of k_gammatone_fast.cu) for
+// those of a warp's 32 frames that `which` names, eight at a time: four lanes
+// a frame, one a stage, each a block of eight samples behind the one before
+// it, so that a sample is four FP64 instructions of the warp (a lane that runs
+// all stages issues 13, and beside another stream's tensor products each
+// waits for the pipe: 200 us in place of 70 a launch of a speech batch).
+// Silence in front of the first sample leaves the state at zero and is
+// passed over.
+__device__ __noinline__ void recurrences(unsigned which, const SpectralFrame *__restrict__ frames, int band,
+                                         const double *__restrict__ hann, int window, const FastBandCoeffs &k) {
+    constexpr int B = 8;
+    const int lane = threadIdx.x & 31, q = lane & 3;
+    const double beta = k.beta64[q], nd1 = -k.d1, nd2 = -k.d2;
+    while (which) {
+        unsigned mine = which;
+        for (int g = lane >> 2; g > 0 && mine; --g) mine &= mine - 1;
+        const SpectralFrame fr = frames[mine ? __ffs(mine) - 1 : 0];
+        double p[B], h[B], v[B] = {}, v1 = 0.0, y1 = 0.0, y2 = 0.0, acc = 0.0;
+        auto fetch = [&](int i0) {
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const int i = i0 + j;
+                const bool in = q == 0 && mine && i < window && i >= fr.lo && i < fr.hi;
+                p[j] = in ? __ldg(fr.p + i) : 0.0;
+                h[j] = in ? __ldg(hann + i) : 0.0;
+            }
+        };
+        bool quiet = true;
+        fetch(0);
+        for (int i0 = 0; i0 < window + 3 * B; i0 += B) {  // stage q: samples from i0 - B q
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const double before = __shfl_up_sync(0xffffffffu, v[j], 1);
+                v[j] = q ? before : p[j] * h[j];
+                quiet = quiet && (q || v[j] == 0.0);
+            }
+            fetch(i0 + B);
+            if (__all_sync(0xffffffffu, quiet)) continue;
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const double y = __fma_rn(nd1, y1, __fma_rn(nd2, y2, __fma_rn(beta, v1, v[j])));
+                v1 = v[j];
+                y2 = y1;
+                y1 = y;
+                v[j] = y;
+                if (i0 - B * q + j < window) acc = __fma_rn(y, y, acc);
+            }
+        }
+        if (q == 3 && mine) fr.out[band * fr.stride] = sqrt(acc / (double)window) * k.post64;
+        for (int g = 0; g < 8 && which; ++g) which &= which - 1;
     }
-    return sqrt(acc / (double)window) * k.post64;
 }
 
 // A thread per frame and band. Where nearly all of the response's energy
@@ -402,7 +437,7 @@ __device__ __noinline__ double recurrence(const SpectralFrame &fr, const double 
 // those cells, and those that are not finite, take the recurrence. At 2^-6 of
 // the energy the difference has lost two digits of 1e-16, still less than the
 // recurrence loses at its worst (3.5e-13); below it a few cells per onset
-// remain, ~25 us of one thread's steps at 3840 samples (a pair's time and a
+// remain (a pair's time and a
 // batch's were the same within the runs' noise with the line at 2^-10).
 constexpr double kCancelled = 1.0 / 64;
 __global__ void __launch_bounds__(128) finish_kernel(const SpectralFrame *__restrict__ frames, int nframes,
@@ -413,21 +448,21 @@ __global__ void __launch_bounds__(128) finish_kernel(const SpectralFrame *__rest
                                                      const double *__restrict__ hann, int window,
                                                      const FastBandCoeffs *__restrict__ coeffs) {
     const int f = blockIdx.x * 128 + threadIdx.x, band = blockIdx.y;
-    if (f >= nframes) return;
+    const bool inside = f < nframes;
     double total = 0.0, tail = 0.0;
-    for (int s = 0; s < splits; ++s) total += power_part[(int64_t)(s * nbp + band) * cap + f];
+    for (int s = 0; s < splits && inside; ++s) total += power_part[(int64_t)(s * nbp + band) * cap + f];
     const int slot = quad_slot[band >> 2], segs = quad_segs[band >> 2];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         double c = 0.0;
-        for (int s = 0; s < segs; ++s) c += tail_part[(int64_t)((slot + s) * 32 + (band & 3) * 8 + j) * cap + f];
+        for (int s = 0; s < segs && inside; ++s) c += tail_part[(int64_t)((slot + s) * 32 + (band & 3) * 8 + j) * cap + f];
         tail = __fma_rn(c, c, tail);
     }
     const double e = total - tail;
-    const SpectralFrame fr = frames[f];
-    double rms = sqrt(e);
-    if (!(e > kCancelled * total && e <= 1.7976931348623157e308)) rms = total == 0.0 ? 0.0 : recurrence(fr, hann, window, coeffs[band]);
-    fr.out[band * fr.stride] = rms;
+    const bool kept = e > kCancelled * total && e <= 1.7976931348623157e308;
+    if (inside && (kept || total == 0.0)) frames[f].out[band * frames[f].stride] = kept ? sqrt(e) : 0.0;
+    const unsigned rest = __ballot_sync(0xffffffffu, inside && !kept && total != 0.0);
+    if (rest) recurrences(rest, frames + (f & ~31), band, hann, window, coeffs[band]);
 }
 
 constexpr int kChunk = 2048;  // frames of a launch
