@@ -498,7 +498,7 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
                + 16 * n_global + 16 * 1024                     // lag search and argmax parts
                + 8 * al                                        // aligned, scaled degraded signal
                + 8 * NB * (2 * nfr + 2 * nfd + 4 * width)      // spectrograms, prepared copies, plane
-               + np * (8 * 4 * NB * P + 24 * nfd + 8 * (3 * NB + 1) + 16)  // terms, table, DP, stats
+               + np * (8 * 3 * NB * P + 24 * nfd + 8 * (3 * NB + 1) + 16)  // terms, table, DP, stats
                + np * (16 * n_slice + 8 * 4 * NB * (2 * P + 2) + 256);     // realignment slices
     b += b / 4 + (size_t(1) << 20);  // job tables, tiles, rounding slack
     return b;
@@ -899,7 +899,8 @@ struct PairState {
     host::Search search;
     size_t width = 0;
     double *deg_al = nullptr, *ref_raw = nullptr, *deg_raw = nullptr, *ref_prep = nullptr, *deg_prep = nullptr;
-    double *pad = nullptr, *mu = nullptr, *dms = nullptr, *sds = nullptr, *terms = nullptr, *sims = nullptr;
+    double *pad = nullptr, *terms = nullptr, *sims = nullptr;
+    double2 *plane = nullptr;
     double *dp = nullptr;
     int64_t *bt = nullptr, *offs = nullptr;
     uint8_t *valid = nullptr;
@@ -1126,12 +1127,12 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     std::vector<PrepJob> prep_jobs;
     std::vector<PlaneJob> plane_jobs;
     std::vector<RefTermsJob> term_jobs;
-    std::vector<TableTask> table_rows;  // one per patch: offsets [off0, hi]
+    std::vector<TableTask> table_rows;  // one per patch
     std::vector<DpJob> dp_jobs;
     std::vector<int64_t> all_lohi;  // per DP job: its patches' lo, then hi
     std::vector<size_t> lohi_at;
     std::vector<StatsJob> stat_jobs;
-    int max_width = 0;
+    int max_width = 0, max_offsets = 0;
     size_t npatches = 0;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
@@ -1187,11 +1188,9 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         s.ref_prep = arena_.alloc_n<double>(NB * s.nf_ref);
         s.deg_prep = arena_.alloc_n<double>(NB * s.nf_deg);
         const size_t plane = NB * s.width;
-        s.pad = arena_.alloc_n<double>(4 * plane);
-        s.mu = s.pad + plane;
-        s.dms = s.mu + plane;
-        s.sds = s.dms + plane;
-        s.terms = arena_.alloc_n<double>(np * 4 * NB * P);
+        s.pad = arena_.alloc_n<double>(plane);
+        s.plane = arena_.alloc_n<double2>(plane);
+        s.terms = arena_.alloc_n<double>(np * ref_terms_count(NB, P));
         s.sims = arena_.alloc_n<double>(np * s.nf_deg);
         s.dp = arena_.alloc_n<double>(np * s.nf_deg);
         s.bt = arena_.alloc_n<int64_t>(np * s.nf_deg);
@@ -1207,17 +1206,18 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         spec_jobs.push_back(SpecJob{VSig{s.deg_al, 0, s.al.len, s.al.len}, (int64_t)s.nf_deg, s.deg_raw});
         s.trace.n_rms += NB * (s.nf_ref + s.nf_deg);
         prep_jobs.push_back(PrepJob{s.ref_raw, s.deg_raw, s.ref_prep, s.deg_prep, (int32_t)s.nf_ref, (int32_t)s.nf_deg});
-        plane_jobs.push_back(PlaneJob{s.deg_prep, (int32_t)s.nf_deg, (int32_t)s.width, s.pad, s.mu, s.dms, s.sds,
+        plane_jobs.push_back(PlaneJob{s.deg_prep, (int32_t)s.nf_deg, (int32_t)s.width, s.pad, s.plane,
                                       opt_.form != kFormExact ? 1 : 0});
         lohi_at.push_back(all_lohi.size());
         all_lohi.insert(all_lohi.end(), s.search.lo.begin(), s.search.lo.end());
         all_lohi.insert(all_lohi.end(), s.search.hi.begin(), s.search.hi.end());
         for (size_t p = 0; p < np; ++p) {
-            double *terms = s.terms + p * 4 * NB * P;
+            double *terms = s.terms + p * ref_terms_count(NB, P);
             term_jobs.push_back(RefTermsJob{s.ref_prep, (int32_t)s.nf_ref, (int32_t)s.idx[p], terms,
                                             opt_.form != kFormExact ? 1 : 0});
-            table_rows.push_back(TableTask{terms, s.pad, s.mu, s.dms, s.sds, (int32_t)s.width,
-                                           (int32_t)s.search.lo[p], (int32_t)s.search.hi[p], s.sims + p * s.nf_deg});
+            table_rows.push_back(TableTask{terms, s.pad, s.plane, (int32_t)s.width, (int32_t)s.search.lo[p],
+                                           (int32_t)s.search.hi[p], s.sims + p * s.nf_deg});
+            max_offsets = std::max(max_offsets, (int)(s.search.hi[p] - s.search.lo[p] + 1));
             s.trace.n_cells += (uint64_t)(s.search.hi[p] - s.search.lo[p] + 1) * NB * P;
             double *ms = s.mstats + p * (3 * NB + 1);
             stat_jobs.push_back(StatsJob{s.ref_prep, (int32_t)s.nf_ref, (int32_t)s.idx[p], s.deg_prep,
@@ -1246,18 +1246,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     const DpJob *d_dp = upload(dp_jobs);
     const StatsJob *d_stats = upload(stat_jobs);
     const bool fast_cells = opt_.form != kFormExact;
-    auto upload_tasks = [&](int w) {
-        std::vector<TableTask> tasks;
-        for (const TableTask &row : table_rows)
-            for (int64_t off0 = row.off0; off0 <= row.hi; off0 += w) {
-                TableTask t = row;
-                t.off0 = (int32_t)off0;
-                tasks.push_back(t);
-            }
-        return std::make_pair((const TableTask *)upload(tasks), (int)tasks.size());
-    };
-    const std::vector<int> widths = table_width_candidates((int)P);
-    std::map<int, std::pair<const TableTask *, int>> tasks{{widths[0], upload_tasks(widths[0])}};
+    const TableTask *d_table = upload(table_rows);
     flush_uploads();
     if (nscale) launch_scale(d_scale, nscale, max_al, stream_);
     record(events_[2]);
@@ -1268,14 +1257,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     record(events_[4]);
     launch_plane(d_planes, (int)plane_jobs.size(), nbi, max_width, stream_);
     launch_ref_terms(d_terms, (int)term_jobs.size(), nbi, (int)P, stream_);
-    if (!table_rows.empty()) {
-        auto launch_width = [&](int w) {
-            if (!tasks.count(w)) tasks[w] = upload_tasks(w);
-            flush_uploads();
-            launch_table(tasks[w].first, tasks[w].second, nbi, (int)P, fast_cells, w, stream_);
-        };
-        launch_width(tuned(kTuneTable, fast_cells ? 1 : 0, nbi, widths, launch_width, stream_));
-    }
+    launch_table(d_table, (int)table_rows.size(), max_offsets, nbi, (int)P, fast_cells, stream_);
     launch_dp(d_dp, (int)dp_jobs.size(), stream_);
     launch_stats(d_stats, (int)stat_jobs.size(), nbi, stream_);
     char *h_match = static_cast<char *>(pinned_.alloc(match_bytes));

@@ -220,7 +220,6 @@ private:
     // shape c on st), then reused; candidates[0] when autotuning is off.
     enum TuneKernel {
         kTuneGammatone = 0,
-        kTuneTable = 1,
         kTuneLagColumns = 2
     };
     // VISQOL_TUNE_<kernel> may fix the shape to one of `allowed` (default:

@@ -3,12 +3,9 @@
 //
 // Table: NSIM of every reference patch at every degraded offset in its
 // search window (reference src/accel.zig:126-146, measureSimilarityAt
-// src/nsim.zig:364-424). One thread owns one (patch, offset) and walks the
-// patch's cells in row-major order, so its serial sum is the CPU's order.
-// The threads of a CTA share one reference patch: its values and its
-// precomputed terms (3x3 mean, mean², variance) sit in shared memory and
-// are read as broadcasts; the degraded plane's terms come from global
-// memory, and neighbouring threads read neighbouring offsets (coalesced).
+// src/nsim.zig:364-424). A lane owns an offset, a warp a pair of the patch's
+// band rows at a time (table_kernel). Neighbouring lanes read neighbouring
+// offsets of the degraded plane (coalesced) and the same reference terms.
 // Interior patch columns reuse the plane's terms, whose 3x3 neighbourhood
 // is the patch's; the two edge columns are recomputed with the patch's
 // replicate padding, as the CPU does.
@@ -27,8 +24,8 @@ namespace {
 __device__ inline double signed_root(double v) { return v < 0.0 ? -sqrt(-v) : sqrt(v); }
 
 // Degraded plane of one pair: the prepared spectrogram zero-padded to
-// `width` frames, its 3x3 mean, mean² and variance (reference
-// src/nsim.zig:236-263). out arrays are nb x width.
+// `width` frames, its 3x3 mean and variance (reference
+// src/nsim.zig:236-263).
 __global__ void __launch_bounds__(256) plane_kernel(const PlaneJob *__restrict__ jobs, int nb) {
     const PlaneJob job = jobs[blockIdx.y];
     const int w = job.width, nf = job.nf;
@@ -46,14 +43,12 @@ __global__ void __launch_bounds__(256) plane_kernel(const PlaneJob *__restrict__
                                  p21 * p21, p22 * p22);
         const double dms = mu * mu;
         job.pad[e] = p11;
-        job.mu[e] = mu;
-        job.dms[e] = dms;
-        job.sds[e] = job.roots ? signed_root(csq - dms) : csq - dms;
+        job.terms[e] = make_double2(mu, job.roots ? signed_root(csq - dms) : csq - dms);
     }
 }
 
 // Reference-patch terms (reference precomputeRef, src/nsim.zig:318-329):
-// out[4][nb][P] = {patch values, 3x3 mean, mean², conv(x²) - mean²}.
+// pairs {3x3 mean, conv(x²) - mean²}, then the patch values.
 __global__ void __launch_bounds__(256) ref_terms_kernel(const RefTermsJob *__restrict__ jobs, int nb, int P) {
     const RefTermsJob job = jobs[blockIdx.y];
     const int total = nb * P;
@@ -69,19 +64,17 @@ __global__ void __launch_bounds__(256) ref_terms_kernel(const RefTermsJob *__res
         const double csq = taps9(p00 * p00, p01 * p01, p02 * p02, p10 * p10, p11 * p11, p12 * p12, p20 * p20,
                                  p21 * p21, p22 * p22);
         const double rms = mu * mu;
-        job.out[e] = p11;
-        job.out[total + e] = mu;
-        job.out[2 * total + e] = rms;
-        job.out[3 * total + e] = job.roots ? signed_root(csq - rms) : csq - rms;
+        reinterpret_cast<double2 *>(job.out)[e] = make_double2(mu, job.roots ? signed_root(csq - rms) : csq - rms);
+        job.out[2 * total + e] = p11;
     }
 }
 
-constexpr int kTableThreads = 128;  // default offsets per CTA
-
-// The fast forms' cell arithmetic: the 3x3 window as an FMA chain and the
-// cell's two quotients as one, (2 mr md + c1)(srd + c3) /
-// ((rms + dms + c1)(sqrt(srs sds) + c3)), about half the f64 instructions of
-// the exact cell; values agree with it to a few ulp.
+// The fast forms' 3x3 window as an FMA chain and their quotient: the cell's
+// two quotients as one, (2 mr md + c1)(srd + c3) / ((rms + dms + c1)
+// (sqrt(srs sds) + c3)), by a positive denominator with a reciprocal estimate
+// refined by Newton-Raphson iterations (Markstein's refinement: r' = r +
+// r(1 - d r), then q' = q + r'(n - d q)), which agrees with the IEEE quotient
+// to about an ulp.
 __device__ inline double taps9_fma(double a00, double a01, double a02, double a10, double a11, double a12,
                                    double a20, double a21, double a22) {
     double t = kW0 * a00;
@@ -95,100 +88,6 @@ __device__ inline double taps9_fma(double a00, double a01, double a02, double a1
     return __fma_rn(kW0, a22, t);
 }
 
-// sr, sd: signed roots of the reference and degraded variances.
-__device__ inline double sim_cell_fast(double mr, double rms, double sr, double md, double dms, double sd,
-                                       double crd) {
-    const double mrd = mr * md;
-    const double srd = crd - mrd;
-    const double q = sr * sd;
-    const double sden = q < 0.0 ? kC3 : fabs(q) + kC3;
-    return (__fma_rn(2.0, mrd, kC1) * (srd + kC3)) / ((rms + dms + kC1) * sden);
-}
-
-template <bool kFast>
-__device__ inline double taps(double a00, double a01, double a02, double a10, double a11, double a12, double a20,
-                              double a21, double a22) {
-    return kFast ? taps9_fma(a00, a01, a02, a10, a11, a12, a20, a21, a22)
-                 : taps9(a00, a01, a02, a10, a11, a12, a20, a21, a22);
-}
-
-// One thread per (patch, offset); CTA = one patch x 128 offsets.
-template <bool kFast, int kThreads>
-__global__ void __launch_bounds__(kThreads) table_kernel(const TableTask *__restrict__ tasks, int nb, int P) {
-    extern __shared__ double sm[];
-    const TableTask t = tasks[blockIdx.x];
-    const int total = nb * P;
-    for (int e = threadIdx.x; e < 4 * total; e += blockDim.x) sm[e] = t.ref_terms[e];
-    __syncthreads();
-    const int64_t off = t.off0 + threadIdx.x;
-    if (off > t.hi) return;
-    const double *rv = sm, *mr = sm + total, *rms = sm + 2 * total, *srs = sm + 3 * total;
-    const int w = t.width;
-    const double *pad = t.pad, *mu = t.mu, *dmsp = t.dms, *sdsp = t.sds;
-    double sum = 0.0;
-    for (int r = 0; r < nb; ++r) {
-        const int rm = r == 0 ? 0 : r - 1, rp = r + 1 >= nb ? nb - 1 : r + 1;
-        const double *pm = pad + (int64_t)rm * w + off, *p0 = pad + (int64_t)r * w + off,
-                     *pp = pad + (int64_t)rp * w + off;
-        const double *qm = rv + rm * P, *q0 = rv + r * P, *qp = rv + rp * P;
-        // ref x deg products of the 3 rows, columns (c-1, c, c+1) clamped
-        // to the patch; slid along c.
-        double am = qm[0] * pm[0], a0 = q0[0] * p0[0], ap = qp[0] * pp[0];  // column cm
-        double bm = am, b0 = a0, bp = ap;                                   // column c
-        for (int c = 0; c < P; ++c) {
-            const int cp = c + 1 >= P ? P - 1 : c + 1;
-            const double cm_ = qm[cp] * pm[cp], c0 = q0[cp] * p0[cp], cpp = qp[cp] * pp[cp];
-            // Taps.row over the patch's ref x deg products.
-            const double crd = taps<kFast>(am, bm, cm_, a0, b0, c0, ap, bp, cpp);
-            double md, dms, sds;
-            if (c == 0 || c == P - 1) {
-                const int cmi = c == 0 ? 0 : c - 1;
-                const double d00 = pm[cmi], d01 = pm[c], d02 = pm[cp];
-                const double d10 = p0[cmi], d11 = p0[c], d12 = p0[cp];
-                const double d20 = pp[cmi], d21 = pp[c], d22 = pp[cp];
-                md = taps<kFast>(d00, d01, d02, d10, d11, d12, d20, d21, d22);
-                const double cdsq = taps<kFast>(d00 * d00, d01 * d01, d02 * d02, d10 * d10, d11 * d11, d12 * d12,
-                                                d20 * d20, d21 * d21, d22 * d22);
-                dms = md * md;
-                sds = kFast ? signed_root(cdsq - dms) : cdsq - dms;
-            } else {
-                const int64_t pi = (int64_t)r * w + off + c;
-                md = mu[pi];
-                dms = dmsp[pi];
-                sds = sdsp[pi];
-            }
-            const int ri = r * P + c;
-            sum += kFast ? sim_cell_fast(mr[ri], rms[ri], srs[ri], md, dms, sds, crd)
-                         : sim_cell(mr[ri], rms[ri], srs[ri], md, dms, sds, crd);
-            // slide: column c becomes cm, column cp becomes c
-            am = bm, a0 = b0, ap = bp;
-            bm = cm_, b0 = c0, bp = cpp;
-        }
-    }
-    t.out[off] = sum / (double)(nb * P);
-}
-
-// The table with the patch width P known at compile time (30 in audio
-// mode, 20 in speech mode) and W offsets per CTA. The exact form (kFast
-// false) computes the cells of table_kernel<false, W> with the same
-// operations in the same order; the fast forms (kFast true) compute
-// table_kernel<true, W>'s cells, which need not follow the CPU's order,
-// arranged for throughput:
-//
-// * the degraded plane's rows and the reference terms' rows are streamed
-//   through shared memory, one band row at a time and double-buffered with
-//   asynchronous copies: row r needs the padded spectrogram's rows r-1, r,
-//   r+1 and the 3x3 mean, mean^2 and variance planes' row r over the CTA's
-//   columns [off0, off0 + W + P - 1), and the same rows of the reference
-//   patch's terms (about 18 KB of shared memory per CTA at W = 128, so
-//   that register use, not shared memory, bounds the CTAs per SM);
-// * the 3x3 window of the ref x deg products uses per-column sums (the
-//   window is symmetric: corners, edges, centre), about 7 operations per
-//   cell at dependency depth ~4 instead of a 9-deep FMA chain;
-// * the cell's one quotient divides by a positive denominator with a
-//   reciprocal estimate refined by Newton-Raphson iterations (Markstein's
-//   refinement: r' = r + r(1 - d r), then q' = q + r'(n - d q)), which
-//   agrees with the IEEE quotient to about an ulp.
 __device__ inline double fast_quotient(double n, double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
@@ -198,135 +97,185 @@ __device__ inline double fast_quotient(double n, double d) {
     return __fma_rn(r, __fma_rn(-d, q, n), q);
 }
 
-__device__ inline double sim_cell_quick(double mr, double rms, double sr, double md, double dms, double sd,
-                                        double crd) {
+// sr, sd: signed roots of the reference and degraded variances.
+__device__ inline double sim_cell_quick(double mr, double sr, double md, double sd, double crd) {
     const double mrd = mr * md;
     const double srd = crd - mrd;
     const double q = sr * sd;
     const double sden = q < 0.0 ? kC3 : fabs(q) + kC3;
-    return fast_quotient(__fma_rn(2.0, mrd, kC1) * (srd + kC3), (rms + dms + kC1) * sden);
+    return fast_quotient(__fma_rn(2.0, mrd, kC1) * (srd + kC3), __fma_rn(mr, mr, __fma_rn(md, md, kC1)) * sden);
 }
 
-constexpr int kStageRows = 6;  // pad rows r-1, r, r+1; mu, dms, sds rows r
-
-__device__ inline void cp_async8(double *dst, const double *src, int bytes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+template <bool kFast>
+__device__ inline double taps(double a00, double a01, double a02, double a10, double a11, double a12, double a20,
+                              double a21, double a22) {
+    return kFast ? taps9_fma(a00, a01, a02, a10, a11, a12, a20, a21, a22)
+                 : taps9(a00, a01, a02, a10, a11, a12, a20, a21, a22);
 }
 
-template <bool kFast, int P, int W>
-__global__ void __launch_bounds__(W) table_staged_kernel(const TableTask *__restrict__ tasks, int nb) {
-    extern __shared__ __align__(16) double smf[];
-    constexpr int kSpan = W + P - 1;                        // degraded columns a CTA reads
-    constexpr int kStage = kStageRows * kSpan + kStageRows * P;  // one band row's stage
-    const TableTask t = tasks[blockIdx.x];
-    const int total = nb * P;
-    const int w = t.width;
-    // Row r's stage: the degraded plane's rows (pad r-1, r, r+1; mu, dms, sds
-    // r) over the CTA's columns, then the reference terms' rows (values r-1,
-    // r, r+1; mean, mean^2, variance r) over the patch's P columns.
-    auto fetch = [&](int r, int buf) {
-        const int rm = r == 0 ? 0 : r - 1, rp = r + 1 >= nb ? nb - 1 : r + 1;
-        double *dst = smf + buf * kStage;
-        for (int e = threadIdx.x; e < kStageRows * kSpan; e += W) {
-            const int k = e / kSpan, col = t.off0 + (e - k * kSpan);
-            const int row = k == 0 ? rm : k == 2 ? rp : r;
-            const double *plane = k < 3 ? t.pad : k == 3 ? t.mu : k == 4 ? t.dms : t.sds;
-            const double *src = plane + (int64_t)row * w;
-            const bool in = col < w;
-            cp_async8(dst + e, in ? src + col : src, in ? 8 : 0);
-        }
-        double *tdst = dst + kStageRows * kSpan;
-        for (int e = threadIdx.x; e < kStageRows * P; e += W) {
-            const int k = e / P, c = e - k * P;
-            const int row = k == 0 ? rm : k == 2 ? rp : r;
-            const int term = k < 3 ? 0 : k - 2;  // values, mean, mean^2, variance
-            cp_async8(tdst + e, t.ref_terms + term * total + row * P + c, 8);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    fetch(0, 0);
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    const int64_t off = t.off0 + threadIdx.x;
-    double sum = 0.0;
-    for (int r = 0; r < nb; ++r) {
-        if (r + 1 < nb) fetch(r + 1, (r + 1) & 1);
-        const double *stg = smf + (r & 1) * kStage;
-        const double *st = stg + threadIdx.x;
-        const double *pm = st, *p0 = st + kSpan, *pp = st + 2 * kSpan;
-        const double *mu = st + 3 * kSpan, *dm = st + 4 * kSpan, *sd = st + 5 * kSpan;
-        const double *tr = stg + kStageRows * kSpan;
-        const double *qm = tr, *q0 = tr + P, *qp = tr + 2 * P, *mr = tr + 3 * P, *rms = tr + 4 * P, *srs = tr + 5 * P;
-        if (kFast) {
-            // column sums of the ref x deg products: E = rows r-1 + r+1, M = row r
-            double Ec = qm[0] * pm[0] + qp[0] * pp[0], Mc = q0[0] * p0[0];
-            double Em = Ec, Mm = Mc;
-#pragma unroll
-            for (int c = 0; c < P; ++c) {
-                const int cp = c + 1 < P ? c + 1 : P - 1;
-                double Ep = Ec, Mp = Mc;
-                if (c + 1 < P) {
-                    Ep = qm[cp] * pm[cp] + qp[cp] * pp[cp];
-                    Mp = q0[cp] * p0[cp];
-                }
-                const double crd = __fma_rn(kW2, Mc, __fma_rn(kW1, (Mm + Mp) + Ec, kW0 * (Em + Ep)));
-                double md, dms, sds;
-                if (c == 0 || c == P - 1) {
-                    const int cm = c == 0 ? 0 : c - 1;
-                    const double d00 = pm[cm], d01 = pm[c], d02 = pm[cp];
-                    const double d10 = p0[cm], d11 = p0[c], d12 = p0[cp];
-                    const double d20 = pp[cm], d21 = pp[c], d22 = pp[cp];
-                    md = taps9_fma(d00, d01, d02, d10, d11, d12, d20, d21, d22);
-                    const double cdsq = taps9_fma(d00 * d00, d01 * d01, d02 * d02, d10 * d10, d11 * d11,
-                                                  d12 * d12, d20 * d20, d21 * d21, d22 * d22);
-                    dms = md * md;
-                    sds = signed_root(cdsq - dms);
-                } else {
-                    md = mu[c];
-                    dms = dm[c];
-                    sds = sd[c];
-                }
-                sum += sim_cell_quick(mr[c], rms[c], srs[c], md, dms, sds, crd);
-                Em = Ec, Mm = Mc;
-                Ec = Ep, Mc = Mp;
-            }
-        } else {
-            // exact: the operations and order of table_kernel<false> (the
-            // CPU's cell, src/nsim.zig:293-308, and its row-major sum), with
-            // the operands read from the stage
-            double am = qm[0] * pm[0], a0 = q0[0] * p0[0], ap = qp[0] * pp[0];  // column cm
-            double bm = am, b0 = a0, bp = ap;                                   // column c
-#pragma unroll
-            for (int c = 0; c < P; ++c) {
-                const int cp = c + 1 >= P ? P - 1 : c + 1;
-                const double cm_ = qm[cp] * pm[cp], c0 = q0[cp] * p0[cp], cpp = qp[cp] * pp[cp];
-                const double crd = taps9(am, bm, cm_, a0, b0, c0, ap, bp, cpp);
-                double md, dms, sds;
-                if (c == 0 || c == P - 1) {
-                    const int cmi = c == 0 ? 0 : c - 1;
-                    const double d00 = pm[cmi], d01 = pm[c], d02 = pm[cp];
-                    const double d10 = p0[cmi], d11 = p0[c], d12 = p0[cp];
-                    const double d20 = pp[cmi], d21 = pp[c], d22 = pp[cp];
-                    md = taps9(d00, d01, d02, d10, d11, d12, d20, d21, d22);
-                    const double cdsq = taps9(d00 * d00, d01 * d01, d02 * d02, d10 * d10, d11 * d11, d12 * d12,
-                                              d20 * d20, d21 * d21, d22 * d22);
-                    dms = md * md;
-                    sds = cdsq - dms;
-                } else {
-                    md = mu[c];
-                    dms = dm[c];
-                    sds = sd[c];
-                }
-                sum += sim_cell(mr[c], rms[c], srs[c], md, dms, sds, crd);
-                am = bm, a0 = b0, ap = bp;
-                bm = cm_, b0 = c0, bp = cpp;
-            }
-        }
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        __syncthreads();
+// One patch column of the ref x deg products, of the form's window.
+template <bool kFast>
+struct Column;
+// Exact: rows r-1 .. r+1 with the window's weights applied (outer rows take kW0
+// at the sides and kW1 in the centre, the middle row kW1 and kW2), summed
+// in taps9's order.
+template <>
+struct Column<false> {
+    double a, b, c;
+    __device__ inline void set(double x, double y, double z, double) { a = x, b = y, c = z; }
+    __device__ static inline double upper(const Column &l, const Column &m, const Column &r) {
+        return taps9(l.a, m.a, r.a, l.b, m.b, r.b, l.c, m.c, r.c);
     }
-    if (off <= t.hi) t.out[off] = sum / (double)(nb * P);
+    __device__ static inline double lower(const Column &, const Column &, const Column &) { return 0.0; }
+};
+// Fast: rows r-1 .. r+2, for the windows of rows r and r+1: the outer rows'
+// sum and the middle row of each.
+template <>
+struct Column<true> {
+    double eu, mu, el, ml;
+    __device__ inline void set(double a, double b, double c, double d) { eu = a + c, mu = b, el = b + d, ml = c; }
+    __device__ static inline double window(double el, double em, double er, double ml, double mm, double mr) {
+        return __fma_rn(kW2, mm, __fma_rn(kW1, (ml + mr) + em, kW0 * (el + er)));
+    }
+    __device__ static inline double upper(const Column &l, const Column &m, const Column &r) {
+        return window(l.eu, m.eu, r.eu, l.mu, m.mu, r.mu);
+    }
+    __device__ static inline double lower(const Column &l, const Column &m, const Column &r) {
+        return window(l.el, m.el, r.el, l.ml, m.ml, r.ml);
+    }
+};
+
+constexpr int kTableWarps = 8;
+constexpr int kTableKept = 64;  // exact form: patch columns up to which a row's cells are kept (128 KB a CTA)
+
+__device__ inline void hand_over(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ inline void take_over(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// The table: grid (tiles of 32 offsets, patches), a lane an offset, the
+// patch's band rows to the CTA's warps in turn.
+//
+// Exact form: the CPU adds the cells one by one in row-major order, so a warp
+// keeps a row's cells in shared memory and adds them to the running sum
+// when the row before has been added (a named barrier hands the 32 sums from
+// warp to warp): the serial part is the additions alone, and the cells (two
+// IEEE quotients and a root each) are formed by eight warps at once. Patches
+// too wide to keep run on one warp. The fast forms take rows by pairs (four
+// rows' products instead of six, two independent cells) and add up a warp's
+// cells, then the warps.
+//
+// A cell is ~600 cycles of dependent quotients, roots and sums, so the warps
+// in flight decide a small launch and issue slots (half of them not FP64) a
+// large one: 128 registers for two CTAs an SM; by pairs the exact form has
+// 190 and is slower. Against a thread per patch and offset over all its cells:
+// an exact pair of 16 patches x 497 offsets 312 to 71 us, a fast one of 317
+// offsets 123 to 23 us; lanes' time over 64 fast 10 s pairs 5.5 to 1.9 ms,
+// over 32 exact ones 7.2 to 2.6 ms; 100 patches x 2977 offsets, which filled
+// the chip before, 1.53 to 1.54 ms.
+template <bool kFast, int kP>
+__global__ void __launch_bounds__(kTableWarps * 32, 2) table_kernel(const TableTask *__restrict__ tasks,
+                                                                      int nb, int P_) {
+    const int P = kP ? kP : P_;
+    extern __shared__ double cells_sm[];  // exact form: [warp][P][32]
+    __shared__ double sums_sm[kTableWarps][32];
+    const TableTask t = tasks[blockIdx.y];
+    const int off0 = t.lo + blockIdx.x * 32;
+    if (off0 > t.hi) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int off = min(off0 + lane, t.hi);
+    constexpr int step = kFast ? 2 : 1;
+    const int items = (nb + step - 1) / step;
+    const int w = t.width;
+    const double2 *rterms = reinterpret_cast<const double2 *>(t.ref_terms);
+    const double *rvals = t.ref_terms + 2 * (int64_t)nb * P;
+    double *mine = cells_sm + (int64_t)warp * P * 32 + lane;
+    double sum = 0.0;
+    for (int item = warp; item < items; item += warps) {
+        const int r = item * step;
+        const bool two = kFast && r + 1 < nb;
+        const int rows[4] = {max(r - 1, 0), r, min(r + 1, nb - 1), min(r + 2, nb - 1)};
+        const double *q[4], *p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            q[k] = rvals + (int64_t)rows[k] * P;
+            p[k] = t.pad + (int64_t)rows[k] * w + off;
+        }
+        const double2 *ru = rterms + (int64_t)r * P, *rl = rterms + (int64_t)rows[2] * P;
+        const double2 *du = t.terms + (int64_t)r * w + off, *dl = t.terms + (int64_t)rows[2] * w + off;
+        auto product = [&](int k, int c) { return __ldg(q[k] + c) * __ldg(p[k] + c); };
+        auto column = [&](int c) {
+            Column<kFast> v;
+            v.set(product(0, c), product(1, c), product(2, c), kFast ? product(3, c) : 0.0);
+            return v;
+        };
+        // the edge columns' mean and variance, with the patch's padding
+        auto edge = [&](const double *pm, const double *p0, const double *pp, int c) {
+            const int cm = max(c - 1, 0), cp = min(c + 1, P - 1);
+            const double d00 = pm[cm], d01 = pm[c], d02 = pm[cp];
+            const double d10 = p0[cm], d11 = p0[c], d12 = p0[cp];
+            const double d20 = pp[cm], d21 = pp[c], d22 = pp[cp];
+            const double md = taps<kFast>(d00, d01, d02, d10, d11, d12, d20, d21, d22);
+            const double sq = taps<kFast>(d00 * d00, d01 * d01, d02 * d02, d10 * d10, d11 * d11, d12 * d12, d20 * d20,
+                                          d21 * d21, d22 * d22);
+            const double var = sq - md * md;
+            return make_double2(md, kFast ? signed_root(var) : var);
+        };
+        auto cell = [&](double2 ref, double2 deg, double crd) {
+            return kFast ? sim_cell_quick(ref.x, ref.y, deg.x, deg.y, crd)
+                         : sim_cell(ref.x, ref.x * ref.x, ref.y, deg.x, deg.x * deg.x, deg.y, crd);
+        };
+        auto put = [&](int c, double u, double l) {
+            if (kFast)
+                sum += two ? u + l : u;
+            else if (warps == 1)
+                sum += u;
+            else
+                mine[c * 32] = u;
+        };
+        auto lower = [&](double2 deg, int c, const Column<kFast> &left, const Column<kFast> &mid, const Column<kFast> &right) {
+            return kFast ? cell(__ldg(rl + c), deg, Column<kFast>::lower(left, mid, right)) : 0.0;
+        };
+        Column<kFast> left = column(0), mid = left;
+        double2 mu = edge(p[0], p[1], p[2], 0), ml = kFast ? edge(p[1], p[2], p[3], 0) : mu;
+#pragma unroll (kP && !kFast ? 5 : 3)
+        for (int c = 0; c + 1 < P; ++c) {  // (unrolled: the columns' registers rotate without moves)
+            const Column<kFast> right = column(c + 1);
+            const double2 nu = __ldg(du + c + 1), nl = kFast ? __ldg(dl + c + 1) : nu;
+            put(c, cell(__ldg(ru + c), mu, Column<kFast>::upper(left, mid, right)),
+                lower(ml, c, left, mid, right));
+            left = mid;
+            mid = right;
+            mu = nu;
+            ml = nl;
+        }
+        if (P > 1) {
+            mu = edge(p[0], p[1], p[2], P - 1);
+            ml = kFast ? edge(p[1], p[2], p[3], P - 1) : mu;
+        }
+        put(P - 1, cell(__ldg(ru + P - 1), mu, Column<kFast>::upper(left, mid, mid)),
+            lower(ml, P - 1, left, mid, mid));
+        if (!kFast && warps > 1) {
+            if (item > 0) {
+                take_over(1 + warp);
+                sum = sums_sm[0][lane];
+            }
+#pragma unroll 4
+            for (int c = 0; c < P; ++c) sum += mine[c * 32];
+            if (item + 1 < items) {
+                sums_sm[0][lane] = sum;
+                __threadfence_block();
+                hand_over(1 + (warp + 1) % warps);
+            }
+        }
+    }
+    if (kFast) {
+        sums_sm[warp][lane] = sum;
+        __syncthreads();
+        if (warp) return;
+        for (int k = 1; k < warps; ++k) sum += sums_sm[k][lane];
+    } else if (warp != (items - 1) % warps) {
+        return;
+    }
+    if (off0 + lane <= t.hi) t.out[off] = sum / (double)(nb * P);
 }
 
 // Per-band statistics of one patch pair, one thread per band row
@@ -440,78 +389,40 @@ void launch_ref_terms(const RefTermsJob *d_jobs, int njobs, int nb, int P, cudaS
     launch_counter() += 1;
 }
 
-int table_offsets_per_cta() { return kTableThreads; }
-
-std::vector<int> table_width_candidates(int P) {
-    // widths the staged kernels have for the audio and speech patch widths;
-    // 64 would fall back to the unstaged kernel
-    if (P == 30 || P == 20) return {128, 256};
-    return {128, 64, 256};
-}
-
 void nsim_init_attributes() {
-    cudaFuncSetAttribute(table_kernel<false, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(table_kernel<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(table_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(table_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(table_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(table_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-#define VQB_STAGED_ATTR(F, PP, W) \
-    cudaFuncSetAttribute(table_staged_kernel<F, PP, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    VQB_STAGED_ATTR(true, 30, 128)
-    VQB_STAGED_ATTR(true, 30, 256)
-    VQB_STAGED_ATTR(true, 20, 128)
-    VQB_STAGED_ATTR(true, 20, 256)
-    VQB_STAGED_ATTR(false, 30, 128)
-    VQB_STAGED_ATTR(false, 30, 256)
-    VQB_STAGED_ATTR(false, 20, 128)
-    VQB_STAGED_ATTR(false, 20, 256)
-#undef VQB_STAGED_ATTR
+    const int bytes = kTableWarps * kTableKept * 32 * (int)sizeof(double);
+    cudaFuncSetAttribute(table_kernel<false, 30>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(table_kernel<false, 20>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaFuncSetAttribute(table_kernel<false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-void launch_table(const TableTask *d_tasks, int ntasks, int nb, int P, bool fast, int width, cudaStream_t s) {
-    if (ntasks <= 0) return;
-    const size_t smem = (size_t)4 * nb * P * sizeof(double);
-    if ((P == 30 || P == 20) && (width == 128 || width == 256)) {
-        const size_t staged = (size_t)2 * kStageRows * ((width + P - 1) + P) * sizeof(double);
-#define VQB_TABLE_STAGED(F, PP, W) table_staged_kernel<F, PP, W><<<ntasks, W, staged, s>>>(d_tasks, nb);
-#define VQB_TABLE_STAGED_P(F)            \
-    if (P == 30) {                       \
-        if (width == 256) {              \
-            VQB_TABLE_STAGED(F, 30, 256) \
-        } else {                         \
-            VQB_TABLE_STAGED(F, 30, 128) \
-        }                                \
-    } else {                             \
-        if (width == 256) {              \
-            VQB_TABLE_STAGED(F, 20, 256) \
-        } else {                         \
-            VQB_TABLE_STAGED(F, 20, 128) \
-        }                                \
-    }
-        if (fast) {
-            VQB_TABLE_STAGED_P(true)
-        } else {
-            VQB_TABLE_STAGED_P(false)
-        }
-#undef VQB_TABLE_STAGED_P
-#undef VQB_TABLE_STAGED
+void launch_table(const TableTask *d_tasks, int ntasks, int max_offsets, int nb, int P, bool fast, cudaStream_t s) {
+    const unsigned tiles = (unsigned)((max_offsets + 31) / 32);
+    const bool kept = !fast && P <= kTableKept;
+    const unsigned threads = fast || kept ? kTableWarps * 32 : 32;
+    const size_t smem = kept ? (size_t)kTableWarps * P * 32 * sizeof(double) : 0;
+    for (int t0 = 0; t0 < ntasks; t0 += 65535) {
+        const dim3 grid(tiles, (unsigned)std::min(ntasks - t0, 65535));
+        const TableTask *t = d_tasks + t0;
+        // (the patch widths of the two modes as constants: loads at fixed
+        // distances; 3.06 to 2.64 ms of a batch of 32 exact audio pairs)
+        if (fast && P == 30)
+            table_kernel<true, 30><<<grid, threads, smem, s>>>(t, nb, P);
+        else if (fast)
+            table_kernel<true, 0><<<grid, threads, smem, s>>>(t, nb, P);
+        else if (P == 30)
+            table_kernel<false, 30><<<grid, threads, smem, s>>>(t, nb, P);
+        else if (P == 20)
+            table_kernel<false, 20><<<grid, threads, smem, s>>>(t, nb, P);
+        else
+            table_kernel<false, 0><<<grid, threads, smem, s>>>(t, nb, P);
         launch_counter() += 1;
-        return;
     }
-#define VQB_TABLE(W)                                                             \
-    if (fast)                                                                    \
-        table_kernel<true, W><<<ntasks, W, smem, s>>>(d_tasks, nb, P);           \
-    else                                                                         \
-        table_kernel<false, W><<<ntasks, W, smem, s>>>(d_tasks, nb, P);
-    if (width == 64) {
-        VQB_TABLE(64)
-    } else if (width == 256) {
-        VQB_TABLE(256)
-    } else {
-        VQB_TABLE(128)
-    }
-#undef VQB_TABLE
+}
+
+void launch_stats(const StatsJob *d_jobs, int njobs, int nb, cudaStream_t s) {
+    if (njobs <= 0) return;
+    stats_kernel<<<njobs, 32, 0, s>>>(d_jobs, nb);
     launch_counter() += 1;
 }
 
@@ -519,12 +430,6 @@ void launch_fast_quotient(const double *num, const double *den, double *out, siz
     if (count == 0) return;
     const size_t blocks = std::min<size_t>((count + 255) / 256, 4096);
     quotient_kernel<<<(unsigned)blocks, 256, 0, s>>>(num, den, out, count);
-    launch_counter() += 1;
-}
-
-void launch_stats(const StatsJob *d_jobs, int njobs, int nb, cudaStream_t s) {
-    if (njobs <= 0) return;
-    stats_kernel<<<njobs, 32, 0, s>>>(d_jobs, nb);
     launch_counter() += 1;
 }
 

@@ -15,25 +15,30 @@ namespace vqb {
 struct PlaneJob {
     const double *spec;  // prepared degraded spectrogram, nb x nf
     int32_t nf, width;
-    double *pad, *mu, *dms, *sds;  // nb x width each
-    int32_t roots;  // fast forms: sds holds the signed square root of the variance
+    double *pad;     // nb x width
+    double2 *terms;  // nb x width {3x3 mean, variance}
+    int32_t roots;   // fast forms: the signed square root of the variance
 };
 
 // Reference-patch terms: spec columns [col, col+P) of a prepared
-// spectrogram with nf frames; out is 4 x nb x P.
+// spectrogram with nf frames; out is ref_terms_count(nb, P) doubles: nb x P
+// pairs {3x3 mean, variance}, then the nb x P values.
 struct RefTermsJob {
     const double *spec;
     int32_t nf, col;
-    double *out;
-    int32_t roots;  // fast forms: the variance term holds its signed square root
+    double *out;  // 16-byte aligned
+    int32_t roots;  // fast forms: the signed square root of the variance
 };
+inline size_t ref_terms_count(size_t nb, size_t P) { return (3 * nb * P + 1) / 2 * 2; }
 
-// NSIM table block: offsets [off0, min(off0+127, hi)] of one patch.
+// NSIM of one reference patch at the degraded offsets [lo, hi]; the plane
+// (PlaneJob) is at least hi + P wide.
 struct TableTask {
-    const double *ref_terms;  // 4 x nb x P
-    const double *pad, *mu, *dms, *sds;
+    const double *ref_terms;  // RefTermsJob::out
+    const double *pad;
+    const double2 *terms;
     int32_t width;
-    int32_t off0, hi;
+    int32_t lo, hi;
     double *out;  // row of the table: out[off]
 };
 
@@ -202,12 +207,8 @@ void launch_log10(const double *x, int64_t n, double *out, cudaStream_t s);
 void nsim_init_attributes();
 void launch_plane(const PlaneJob *d_jobs, int njobs, int nb, int max_width, cudaStream_t s);
 void launch_ref_terms(const RefTermsJob *d_jobs, int njobs, int nb, int P, cudaStream_t s);
-int table_offsets_per_cta();
-// fast: the fast forms' cell arithmetic (FMA, one division per cell);
-// width: offsets per CTA, one of table_width_candidates(P) (the first is the
-// default); tasks must be built with the same width.
-std::vector<int> table_width_candidates(int P);
-void launch_table(const TableTask *d_tasks, int ntasks, int nb, int P, bool fast, int width, cudaStream_t s);
+// max_offsets: the largest hi - lo + 1 of the tasks.
+void launch_table(const TableTask *d_tasks, int ntasks, int max_offsets, int nb, int P, bool fast, cudaStream_t s);
 void launch_stats(const StatsJob *d_jobs, int njobs, int nb, cudaStream_t s);
 // The fast forms' NSIM quotient n / d (d > 0, normal) elementwise, for its
 // direct test.

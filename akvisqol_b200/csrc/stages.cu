@@ -263,28 +263,27 @@ int visqol_b200_nsim_table(const double *ref_spec, size_t nf_ref, const double *
         vqb::Engine &e = stage_engine();
         size_t width = nf_deg;
         for (size_t p = 0; p < np; ++p) width = std::max(width, (size_t)hi[p] + patch);
-        DBuf<double> rs(ref_spec, nb * nf_ref), ds(deg_spec, nb * nf_deg), plane(4 * nb * width),
-            terms(np * 4 * nb * patch), sims(np * nf_deg);
+        DBuf<double> rs(ref_spec, nb * nf_ref), ds(deg_spec, nb * nf_deg), pad(nb * width),
+            terms(np * vqb::ref_terms_count(nb, patch)), sims(np * nf_deg);
         VQB_CUDA(cudaMemsetAsync(sims.p, 0, std::max<size_t>(1, np * nf_deg) * sizeof(double), e.stream()));
-        const size_t pl = nb * width;
-        vqb::PlaneJob pj{ds.p, (int32_t)nf_deg, (int32_t)width, plane.p, plane.p + pl, plane.p + 2 * pl, plane.p + 3 * pl,
-                         0};
+        DBuf<double2> plane(nb * width);
+        vqb::PlaneJob pj{ds.p, (int32_t)nf_deg, (int32_t)width, pad.p, plane.p, 0};
         std::vector<vqb::RefTermsJob> tj;
         std::vector<vqb::TableTask> tasks;
+        int max_offsets = 0;
         for (size_t p = 0; p < np; ++p) {
-            double *t = terms.p + p * 4 * nb * patch;
+            double *t = terms.p + p * vqb::ref_terms_count(nb, patch);
             tj.push_back(vqb::RefTermsJob{rs.p, (int32_t)nf_ref, (int32_t)ref_idx[p], t, 0});
-            for (int64_t o = lo[p]; o <= hi[p]; o += vqb::table_offsets_per_cta())
-                tasks.push_back(vqb::TableTask{t, pj.pad, pj.mu, pj.dms, pj.sds, (int32_t)width, (int32_t)o,
-                                               (int32_t)hi[p], sims.p + p * nf_deg});
+            tasks.push_back(vqb::TableTask{t, pj.pad, pj.terms, (int32_t)width, (int32_t)lo[p], (int32_t)hi[p],
+                                           sims.p + p * nf_deg});
+            max_offsets = std::max(max_offsets, (int)(hi[p] - lo[p] + 1));
         }
         DBuf<vqb::PlaneJob> dpj(&pj, 1);
         DBuf<vqb::RefTermsJob> dtj(tj.data(), tj.size());
         DBuf<vqb::TableTask> dtasks(tasks.data(), tasks.size());
         vqb::launch_plane(dpj.p, 1, (int)nb, (int)width, e.stream());
         vqb::launch_ref_terms(dtj.p, (int)tj.size(), (int)nb, (int)patch, e.stream());
-        vqb::launch_table(dtasks.p, (int)tasks.size(), (int)nb, (int)patch, false, vqb::table_offsets_per_cta(),
-                          e.stream());
+        vqb::launch_table(dtasks.p, (int)tasks.size(), max_offsets, (int)nb, (int)patch, false, e.stream());
         VQB_CUDA(cudaStreamSynchronize(e.stream()));
         sims.get(out, np * nf_deg);
     });
