@@ -24,3 +24,13 @@ def test_table(native, oracle, nb, patch, span):
     want = oracle.nsim_table(rs, ds, patch, idx, lo, hi)
     for p in range(idx.size):
         assert np.array_equal(got[p, lo[p]:hi[p] + 1], want[p, lo[p]:hi[p] + 1])
+
+
+@pytest.mark.parametrize("nr,nc", [(32, 32), (9, 33), (32, 64), (21, 65), (1, 31), (8, 97)])
+def test_statistics(native, oracle, nr, nc):
+    rng = np.random.default_rng(nr * 100 + nc)
+    ref, deg = rng.uniform(0, 50, (nr, nc)), rng.uniform(0, 50, (nr, nc))
+    got, want = native.patch_similarity(ref, deg), oracle.patch_similarity(ref, deg)
+    assert got[0] == want[0]
+    for a, b in zip(got[1:], want[1:]):
+        assert np.array_equal(a, b)
