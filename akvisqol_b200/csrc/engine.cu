@@ -486,11 +486,11 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
     const size_t np = nfr / std::max<size_t>(1, P) + 1;
     const size_t n_global = host::fft_size_for(std::max(rl, dl));
     const size_t n_slice = host::fft_size_for(2 * P * H + 2);
-    // FMA forms: a frame's spectrum and partial sums (k_spectral.cu), launches of
-    // at most 2048 frames; the degraded and realigned spectrograms share theirs
-    auto spectral_frames = [](size_t nf) { return std::min<size_t>(nf + 63, 2048); };
-    const size_t spectral = 5 * host::fft_size_for(host::analysis_geometry(sample_rate).window) *
-                            (spectral_frames(nfr) + spectral_frames(std::max(nfd, 2 * np * (P + 2))));
+    // FMA forms: a frame's spectrum and partial sums (k_spectral.cu), up to 2048
+    // frames of 4096 points; the degraded and realigned spectrograms share theirs
+    const size_t points = host::fft_size_for(host::analysis_geometry(sample_rate).window);
+    auto spectral_frames = [&](size_t nf) { return std::min<size_t>(nf + 63, (size_t(1) << 24) / points); };
+    const size_t spectral = 6 * points * (spectral_frames(nfr) + spectral_frames(std::max(nfd, 2 * np * (P + 2))));
     const size_t sums = 2 * serial_sum_scratch(2, (int64_t)std::max(rl, dl)) +
                         serial_sum_scratch((int)(2 * np), (int64_t)(2 * P * H + 2));
     size_t b = 8 * (rl + dl)                                   // inputs

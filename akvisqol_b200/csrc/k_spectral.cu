@@ -33,8 +33,8 @@
 // f64 and 105 with its last two stages in f32. A single 6.4 s pair's call went
 // from 1.34 ms to 0.70, 64 pairs of 10 s from 18.0 ms to 11.2.
 //
-// Three launches over up to 2048 frames (a spectrum row is 33 KB; 2048 rows
-// stay in the L2): spectrum_kernel, a CTA per frame; energy_kernel, a warp per
+// Three launches over up to 2048 48 kHz frames (a spectrum row is 33 KB; 2048
+// rows stay in the L2): spectrum_kernel, a CTA per frame; energy_kernel, a warp per
 // piece and tile of 32 or 64 frames; finish_kernel, the pieces added in order.
 // Every frame's values are formed in the same order whatever its batch.
 #include <algorithm>
@@ -395,35 +395,43 @@ __device__ __noinline__ void recurrences(unsigned which, const SpectralFrame *__
         unsigned mine = which;
         for (int g = lane >> 2; g > 0 && mine; --g) mine &= mine - 1;
         const SpectralFrame fr = frames[mine ? __ffs(mine) - 1 : 0];
-        double p[B], h[B], v[B] = {}, v1 = 0.0, y1 = 0.0, y2 = 0.0, acc = 0.0;
+        const int lo = max(fr.lo, 0), hi = mine ? min(fr.hi, window) : 0;
+        // 32 samples of the frame over its four lanes, read 32 ahead
+        double p[B], h[B], x[B], v[B] = {}, v1 = 0.0, y1 = 0.0, y2 = 0.0, acc = 0.0;
         auto fetch = [&](int i0) {
 #pragma unroll
             for (int j = 0; j < B; ++j) {
-                const int i = i0 + j;
-                const bool in = q == 0 && mine && i < window && i >= fr.lo && i < fr.hi;
+                const int i = i0 + B * q + j;
+                const bool in = i >= lo && i < hi;
                 p[j] = in ? __ldg(fr.p + i) : 0.0;
                 h[j] = in ? __ldg(hann + i) : 0.0;
             }
         };
         bool quiet = true;
         fetch(0);
-        for (int i0 = 0; i0 < window + 3 * B; i0 += B) {  // stage q: samples from i0 - B q
+        for (int i0 = 0; i0 < window + 3 * B; i0 += 4 * B) {
 #pragma unroll
             for (int j = 0; j < B; ++j) {
-                const double before = __shfl_up_sync(0xffffffffu, v[j], 1);
-                v[j] = q ? before : p[j] * h[j];
-                quiet = quiet && (q || v[j] == 0.0);
+                x[j] = p[j] * h[j];
+                quiet = quiet && x[j] == 0.0;
             }
-            fetch(i0 + B);
+            fetch(i0 + 4 * B);
             if (__all_sync(0xffffffffu, quiet)) continue;
+            for (int b = 0; b < 4; ++b) {  // stage q: samples from i0 + B (b - q)
 #pragma unroll
-            for (int j = 0; j < B; ++j) {
-                const double y = __fma_rn(nd1, y1, __fma_rn(nd2, y2, __fma_rn(beta, v1, v[j])));
-                v1 = v[j];
-                y2 = y1;
-                y1 = y;
-                v[j] = y;
-                if (i0 - B * q + j < window) acc = __fma_rn(y, y, acc);
+                for (int j = 0; j < B; ++j) {
+                    const double first = __shfl_sync(0xffffffffu, x[j], b, 4), before = __shfl_up_sync(0xffffffffu, v[j], 1);
+                    v[j] = q ? before : first;
+                }
+#pragma unroll
+                for (int j = 0; j < B; ++j) {
+                    const double y = __fma_rn(nd1, y1, __fma_rn(nd2, y2, __fma_rn(beta, v1, v[j])));
+                    v1 = v[j];
+                    y2 = y1;
+                    y1 = y;
+                    v[j] = y;
+                    if (i0 + B * (b - q) + j < window) acc = __fma_rn(y, y, acc);
+                }
             }
         }
         if (q == 3 && mine) fr.out[band * fr.stride] = sqrt(acc / (double)window) * k.post64;
@@ -465,15 +473,16 @@ __global__ void __launch_bounds__(128) finish_kernel(const SpectralFrame *__rest
     if (rest) recurrences(rest, frames + (f & ~31), band, hann, window, coeffs[band]);
 }
 
-constexpr int kChunk = 2048;  // frames of a launch
 constexpr int kWide = 1024;   // frames from which a tail task takes four bands
 
-int chunk_cap(int nframes) { return (std::min(nframes, kChunk) + 63) / 64 * 64; }
+// Frames of a launch: as many as leave their spectra in the L2 (67 MB).
+int chunk_frames(const SpectralTables &t) { return 2048 << (12 - t.log_m); }
+int chunk_cap(const SpectralTables &t, int nframes) { return (std::min(nframes, chunk_frames(t)) + 63) / 64 * 64; }
 
 }  // namespace
 
 size_t spectral_scratch_count(const SpectralTables &t, int nframes) {
-    return (size_t)chunk_cap(nframes) * (size_t)(t.row + 32 * t.slots + t.nbp * t.splits);
+    return (size_t)chunk_cap(t, nframes) * (size_t)(t.row + 32 * t.slots + t.nbp * t.splits);
 }
 
 int spectral_frame_count(int nframes) { return (nframes + 63) / 64 * 64; }
@@ -484,13 +493,14 @@ void spectral_init_attributes() {
 
 void launch_spectral(const SpectralTables &t, const SpectralDevice &d, const FastBandCoeffs *d_coeffs,
                      const SpectralFrame *d_frames, int nframes, double *d_scratch, cudaStream_t s) {
-    const int cap = chunk_cap(nframes);
+    const int cap = chunk_cap(t, nframes);
     double *power = d_scratch, *tail_part = power + (size_t)cap * t.row,
            *power_part = tail_part + (size_t)cap * 32 * t.slots;
     const int M = 1 << t.log_m;
     const size_t smem = (size_t)(M + M / 16) * sizeof(double2);
-    for (int f0 = 0; f0 < nframes; f0 += kChunk) {
-        const int n = std::min(kChunk, nframes - f0);
+    const int chunk = chunk_frames(t);
+    for (int f0 = 0; f0 < nframes; f0 += chunk) {
+        const int n = std::min(chunk, nframes - f0);
         const SpectralFrame *fr = d_frames + f0;
         if (t.log_m == 12)
             spectrum_kernel<12><<<n, M / 16, smem, s>>>(fr, d.hann, d.twiddles, power, t.row, t.window);
