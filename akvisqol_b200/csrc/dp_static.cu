@@ -22,7 +22,7 @@
 // Sharing: every call on a device uses the same array. Calls that overlap in
 // time on one device (two host threads, say) race on it and must be
 // serialised by the caller. Nothing in the array needs to start at zero:
-// the DP kernel clears its dp and backtrack tables on entry, and the
+// the DP kernel reads no dp or backtrack cell that it has not written, and the
 // offsets and flags are written in full by the backtrack.
 #include <mutex>
 
@@ -47,7 +47,7 @@ constexpr size_t kValidAt = kOffAt + align256(kMaxPatches * sizeof(int64_t));
 constexpr size_t kSimsAt = kValidAt + align256(kMaxPatches);
 constexpr size_t kDpAt = kSimsAt + kMaxCells * sizeof(double);
 constexpr size_t kBtAt = kDpAt + kMaxCells * sizeof(double);
-constexpr size_t kScratchBytes = kBtAt + kMaxCells * sizeof(int64_t);  // ~6.05 MiB
+constexpr size_t kScratchBytes = kBtAt + kMaxCells * sizeof(int32_t);  // ~5.05 MiB
 
 static __device__ __align__(256) unsigned char g_dp_scratch[kScratchBytes];
 
@@ -102,7 +102,7 @@ extern "C" int visqol_b200_dp_static(const double *sims, size_t np, size_t nf_de
     auto *d_valid = reinterpret_cast<uint8_t *>(base + kValidAt);
     auto *d_sims = reinterpret_cast<double *>(base + kSimsAt);
     auto *d_dp = reinterpret_cast<double *>(base + kDpAt);
-    auto *d_bt = reinterpret_cast<int64_t *>(base + kBtAt);
+    auto *d_bt = reinterpret_cast<int32_t *>(base + kBtAt);
 
     const cudaStream_t s = cudaStreamPerThread;
     const vqb::DpJob job{d_sims, d_lo, d_hi, (int32_t)np, (int64_t)nf_deg, d_dp, d_bt, d_off, d_valid};
@@ -111,7 +111,9 @@ extern "C" int visqol_b200_dp_static(const double *sims, size_t np, size_t nf_de
     if (!rc) rc = check(cudaMemcpyAsync(d_hi, hi, np * sizeof(int64_t), cudaMemcpyHostToDevice, s));
     if (!rc) rc = check(cudaMemcpyAsync(d_job, &job, sizeof(job), cudaMemcpyHostToDevice, s));
     if (rc) return rc;
-    vqb::launch_dp(d_job, 1, s);
+    int64_t max_window = 0;
+    for (size_t p = 0; p < np; ++p) max_window = hi[p] - lo[p] + 1 > max_window ? hi[p] - lo[p] + 1 : max_window;
+    vqb::launch_dp(d_job, 1, max_window, s);
     rc = check(cudaGetLastError());
     if (!rc) rc = check(cudaMemcpyAsync(offset, d_off, np * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     if (!rc) rc = check(cudaMemcpyAsync(valid, d_valid, np, cudaMemcpyDeviceToHost, s));

@@ -902,7 +902,8 @@ struct PairState {
     double *pad = nullptr, *terms = nullptr, *sims = nullptr;
     double2 *plane = nullptr;
     double *dp = nullptr;
-    int64_t *bt = nullptr, *offs = nullptr;
+    int32_t *bt = nullptr;
+    int64_t *offs = nullptr;
     uint8_t *valid = nullptr;
     double *mstats = nullptr;
     std::vector<host::Match> matches;
@@ -1193,7 +1194,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         s.terms = arena_.alloc_n<double>(np * ref_terms_count(NB, P));
         s.sims = arena_.alloc_n<double>(np * s.nf_deg);
         s.dp = arena_.alloc_n<double>(np * s.nf_deg);
-        s.bt = arena_.alloc_n<int64_t>(np * s.nf_deg);
+        s.bt = arena_.alloc_n<int32_t>(np * s.nf_deg);
         s.mstats = reinterpret_cast<double *>(d_match) + s.patch0 * per;
         s.offs = reinterpret_cast<int64_t *>(d_match + offs_at) + s.patch0;
         s.valid = reinterpret_cast<uint8_t *>(d_match + valid_at) + s.patch0;
@@ -1258,7 +1259,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     launch_plane(d_planes, (int)plane_jobs.size(), nbi, max_width, stream_);
     launch_ref_terms(d_terms, (int)term_jobs.size(), nbi, (int)P, stream_);
     launch_table(d_table, (int)table_rows.size(), max_offsets, nbi, (int)P, fast_cells, stream_);
-    launch_dp(d_dp, (int)dp_jobs.size(), stream_);
+    launch_dp(d_dp, (int)dp_jobs.size(), max_offsets, stream_);
     launch_stats(d_stats, (int)stat_jobs.size(), nbi, stream_);
     char *h_match = static_cast<char *>(pinned_.alloc(match_bytes));
     d2h(h_match, d_match, match_bytes);

@@ -2,10 +2,22 @@
 //
 // One CTA per pair. Rows (reference patches) are serial. Within a row the
 // CPU keeps a running maximum of the previous row over [prev_lo, slide)
-// with `>=` (ties go to the later offset); that is an inclusive prefix scan
-// under an associative operator, so the CTA forms it as a blocked scan
-// (warp shuffles, then a carry across chunks), then evaluates every slide
-// of the row in parallel. The backtrack is a short serial walk.
+// with `>=` (ties go to the later offset); that is an exclusive prefix scan
+// under an associative operator. A thread takes up to eight consecutive slides
+// of a row, as few as cover it: it scans them itself, a warp scans its
+// threads' totals by shuffles, and every thread adds up the totals of the warps
+// before its own (one barrier). Values are compared as integers, and the two
+// rows in hand stay in shared memory where they fit. Cells outside a row's
+// window are the CPU's zeros: they are not stored but read as such. The
+// backtrack is a short serial walk.
+//
+// Bound by the rows' dependent time. With chunks of 512 slides scanned one
+// behind the other, four barriers a chunk, rows in global memory and the table
+// cleared first, 16 patches x 497 frames took 44 us and 100 x 2997 1180; now
+// 20 and 389. 512 threads take 32 and 460 (barriers), a slide of each round a
+// thread 33 and 635 (more scans).
+#include <algorithm>
+
 #include "device.cuh"
 #include "kernels.h"
 
@@ -13,133 +25,176 @@ namespace vqb {
 
 namespace {
 
-constexpr int kDpThreads = 512;
+constexpr int kDpThreads = 256;
+constexpr int kDpWarps = kDpThreads / 32;
+constexpr int kRowsHeld = 12288;  // slides of a row kept in shared memory (two rows, 192 KB)
 
+// A value and its slide, as integers: key orders like the value (zeros alike;
+// a NaN, which the CPU's `>=` never takes, is empty like the start).
 struct RunMax {
-    double v;
-    int64_t i;  // -1: empty
+    long long key;
+    int32_t i;
 };
-
+__device__ constexpr long long kEmpty = -0x7fffffffffffffffll - 1;
+__device__ inline RunMax element(double v, int s) {
+    const long long b = __double_as_longlong(v + 0.0);
+    return v == v ? RunMax{b ^ (b >> 63 & 0x7fffffffffffffffll), s} : RunMax{kEmpty, -1};
+}
+__device__ inline double value(RunMax x) {  // -inf if empty
+    return x.key == kEmpty ? -INFINITY : __longlong_as_double(x.key ^ (x.key >> 63 & 0x7fffffffffffffffll));
+}
 // Sequential `if (val >= running_max) take` over A then B.
 __device__ inline RunMax combine(RunMax a, RunMax b) {
-    if (b.i < 0) return a;
-    if (a.i < 0) return b;
-    return b.v >= a.v ? b : a;
+    const bool t = b.key >= a.key;
+    return RunMax{t ? b.key : a.key, t ? b.i : a.i};
+}
+__device__ inline RunMax shfl_up(RunMax x, int off) {
+    return RunMax{__shfl_up_sync(0xffffffffu, x.key, off), __shfl_up_sync(0xffffffffu, x.i, off)};
 }
 
-__global__ void __launch_bounds__(kDpThreads) dp_kernel(const DpJob *__restrict__ jobs) {
+// One row of a job: the rows' windows, the previous row's values (slide s at
+// prev[s]) and this row's cells.
+struct Row {
+    int32_t start, end, plo, phi;
+    const double *sims, *prev, *next_sims;  // next_sims: the row after's, or null
+    double *row;
+    int32_t *back;
+};
+
+// Slides c0 .. c0 + kPer x kDpThreads - 1, kPer consecutive ones a thread;
+// carry: the scan up to c0.
+template <int kPer>
+__device__ inline void slides(const Row &r, int c0, RunMax &carry, RunMax *totals) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int s0 = c0 + (int)threadIdx.x * kPer;
+    double p[kPer], sim[kPer];
+    RunMax x{kEmpty, -1}, el[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int s = s0 + k;
+        sim[k] = s >= r.start && s <= r.end ? __ldg(r.sims + s) : 0.0;
+        p[k] = s <= r.end && s <= r.phi ? r.prev[s] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        el[k] = s0 + k <= r.end ? element(p[k], s0 + k) : RunMax{kEmpty, -1};
+        x = combine(x, el[k]);
+    }
+    if (r.next_sims && s0 <= r.end) asm volatile("prefetch.global.L1 [%0];" ::"l"(r.next_sims + s0));
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const RunMax y = shfl_up(x, off);
+        const RunMax z = combine(y, x);
+        x.key = lane >= off ? z.key : x.key;
+        x.i = lane >= off ? z.i : x.i;
+    }
+    if (lane == 31) totals[wid] = x;
+    RunMax run = shfl_up(x, 1);
+    if (lane == 0) run = RunMax{kEmpty, -1};
+    __syncthreads();
+    // what lies before this warp, and all of it
+    RunMax before = carry;
+#pragma unroll
+    for (int w = 0; w < kDpWarps; ++w) {
+        const RunMax t = totals[w];
+        if (w < wid) before = combine(before, t);
+        carry = combine(carry, t);
+    }
+    run = combine(before, run);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int s = s0 + k;
+        const double moved = sim[k] + value(run);
+        const bool stay = p[k] > moved;
+        if (s >= r.start && s <= r.end) {
+            r.row[s] = stay ? p[k] : moved;
+            r.back[s] = stay ? s : run.i;
+        }
+        run = combine(run, el[k]);
+    }
+}
+
+// rows_held: slides of the shared-memory rows (0: every row in global memory).
+__global__ void __launch_bounds__(kDpThreads) dp_kernel(const DpJob *__restrict__ jobs, int rows_held) {
+    extern __shared__ double rows_sm[];  // [2][rows_held]
     const DpJob job = jobs[blockIdx.x];
     const int np = job.np;
     const int64_t cols = job.nf_deg;
-    double *dp = job.dp;
-    int64_t *bt = job.bt;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    __shared__ RunMax warp_tot[kDpThreads / 32];
-    __shared__ RunMax carry_sm;
+    __shared__ RunMax totals[2][kDpWarps];
+    __shared__ double best_v[kDpWarps];
+    __shared__ int32_t best_i[kDpWarps];
 
-    // dp and bt start zeroed, as the CPU's memset (cells outside a row's
-    // window are read as 0 by later rows and by the backtrack).
-    for (int64_t e = tid; e < (int64_t)np * cols; e += blockDim.x) {
-        dp[e] = 0.0;
-        bt[e] = 0;
+    // slide s of row p is row_at(p, ...)[s]
+    auto row_at = [&](int p, int lo, int hi) -> double * {
+        return hi - lo < rows_held ? rows_sm + (p & 1) * rows_held - lo : job.dp + (int64_t)p * cols;
+    };
+    int lo = (int)job.lo[0], hi = (int)job.hi[0];
+    Row r;
+    r.row = row_at(0, lo, hi);
+    for (int s = lo + tid; s <= hi; s += kDpThreads) {
+        r.row[s] = job.sims[s];
+        job.bt[s] = -1;
     }
+    int next_lo = np > 1 ? (int)job.lo[1] : 0, next_hi = np > 1 ? (int)job.hi[1] : 0;
     __syncthreads();
-
-    for (int pi = 0; pi < np; ++pi) {
-        const int64_t start = job.lo[pi], end = job.hi[pi];
-        const double *sims = job.sims + (int64_t)pi * cols;
-        double *row = dp + (int64_t)pi * cols;
-        int64_t *brow = bt + (int64_t)pi * cols;
-        if (pi == 0) {
-            for (int64_t s = start + tid; s <= end; s += blockDim.x) {
-                row[s] = sims[s];
-                brow[s] = -1;
+    int par = 0;
+    for (int pi = 1; pi < np; ++pi) {
+        r.plo = lo, r.phi = hi, r.prev = r.row;
+        r.start = lo = next_lo, r.end = hi = next_hi;
+        if (pi + 1 < np) next_lo = (int)job.lo[pi + 1], next_hi = (int)job.hi[pi + 1];
+        r.sims = job.sims + (int64_t)pi * cols;
+        r.next_sims = pi + 1 < np ? r.sims + cols : nullptr;
+        r.row = row_at(pi, lo, hi);
+        r.back = job.bt + (int64_t)pi * cols;
+        RunMax carry{kEmpty, -1};
+        // (as few slides a thread as cover the row)
+        for (int c0 = r.plo; c0 <= r.end;) {
+            const int left = r.end - c0 + 1;
+            if (left <= kDpThreads) {
+                slides<1>(r, c0, carry, totals[par]);
+                c0 += kDpThreads;
+            } else if (left <= 2 * kDpThreads) {
+                slides<2>(r, c0, carry, totals[par]);
+                c0 += 2 * kDpThreads;
+            } else if (left <= 4 * kDpThreads) {
+                slides<4>(r, c0, carry, totals[par]);
+                c0 += 4 * kDpThreads;
+            } else {
+                slides<8>(r, c0, carry, totals[par]);
+                c0 += 8 * kDpThreads;
             }
-            __syncthreads();
-            continue;
-        }
-        const double *prev = dp + (int64_t)(pi - 1) * cols;
-        const int64_t plo = job.lo[pi - 1];
-        // Running max entering slide s is the scan over prev[plo .. s-1].
-        // Chunks of blockDim elements covering prev[plo .. end-1], the slides
-        // they feed evaluated in the same chunk.
-        RunMax carry{0.0, -1};
-        for (int64_t c0 = plo; c0 <= end; c0 += blockDim.x) {
-            const int64_t e = c0 + tid;  // element index into prev; feeds slide e + 1
-            RunMax x{0.0, -1};
-            if (e < end) x = RunMax{prev[e], e};
-            // inclusive warp scan
-            for (int off = 1; off < 32; off <<= 1) {
-                RunMax y{__shfl_up_sync(0xffffffffu, x.v, off), __shfl_up_sync(0xffffffffu, x.i, off)};
-                if (lane >= off) x = combine(y, x);
-            }
-            if (lane == 31) warp_tot[wid] = x;
-            __syncthreads();
-            if (wid == 0) {
-                RunMax t = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : RunMax{0.0, -1};
-                for (int off = 1; off < 32; off <<= 1) {
-                    RunMax y{__shfl_up_sync(0xffffffffu, t.v, off), __shfl_up_sync(0xffffffffu, t.i, off)};
-                    if (lane >= off) t = combine(y, t);
-                }
-                if (lane < (int)(blockDim.x >> 5)) warp_tot[lane] = t;  // inclusive prefix of warp totals
-            }
-            __syncthreads();
-            RunMax pre = wid > 0 ? warp_tot[wid - 1] : RunMax{0.0, -1};
-            RunMax incl = combine(combine(carry, pre), x);
-            // scan over prev[plo .. e] feeds slide s = e + 1; the first chunk's
-            // slide plo (empty prefix) is handled by the thread with e = plo - 1,
-            // i.e. separately below.
-            const int64_t s = e + 1;
-            if (s >= start && s <= end) {
-                double sim = sims[s];
-                int64_t past = -1;
-                const double rm = incl.i >= 0 ? incl.v : -INFINITY;
-                sim += rm;
-                past = incl.i;
-                const double no_move = prev[s];
-                if (no_move > sim) {
-                    sim = no_move;
-                    past = s;
-                }
-                row[s] = sim;
-                brow[s] = past;
-            }
-            // the chunk's total becomes the carry
-            if (tid == blockDim.x - 1) carry_sm = incl;
-            __syncthreads();
-            carry = carry_sm;
-            __syncthreads();
-        }
-        // Slide `start` when it equals plo: empty running max (-inf, -1).
-        if (tid == 0 && start == plo) {
-            double sim = sims[start] + -INFINITY;
-            int64_t past = -1;
-            const double no_move = prev[start];
-            if (no_move > sim) {
-                sim = no_move;
-                past = start;
-            }
-            row[start] = sim;
-            brow[start] = past;
+            par ^= 1;
         }
         __syncthreads();
     }
 
     // Backtrack from the first maximum of the last row (strict `>`).
+    const int last = np - 1;
+    struct Best {
+        double v;
+        int32_t i;
+    } best{-INFINITY, 0};
+    {
+        for (int s = lo + tid; s <= hi; s += kDpThreads)
+            if (r.row[s] > best.v) best = Best{r.row[s], s};
+    }
+    auto first_max = [](Best a, Best b) { return b.v > a.v || (b.v == a.v && b.v > -INFINITY && b.i < a.i) ? b : a; };
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+        best = first_max(best, Best{__shfl_xor_sync(0xffffffffu, best.v, off), __shfl_xor_sync(0xffffffffu, best.i, off)});
+    if (lane == 0) best_v[wid] = best.v, best_i[wid] = best.i;
+    for (int p = tid; p < np; p += kDpThreads) {
+        job.offset[p] = -1;
+        job.valid[p] = 1;
+    }
+    __syncthreads();
     if (tid == 0) {
-        const int last = np - 1;
-        double best = -INFINITY;
-        int64_t cur = 0;
-        const double *row = dp + (int64_t)last * cols;
-        for (int64_t off = job.lo[last]; off <= job.hi[last]; ++off)
-            if (row[off] > best) best = row[off], cur = off;
-        for (int p = 0; p < np; ++p) {
-            job.offset[p] = -1;
-            job.valid[p] = 1;
-        }
+        for (int k = 1; k < kDpWarps; ++k) best = first_max(best, Best{best_v[k], best_i[k]});
+        int64_t cur = best.i;
         for (int p = last; p >= 0; --p) {
             job.offset[p] = cur;
-            const int64_t back = bt[(int64_t)p * cols + cur];
+            const int64_t back = cur >= job.lo[p] && cur <= job.hi[p] ? job.bt[(int64_t)p * cols + cur] : 0;
             job.valid[p] = back == cur ? 0 : 1;
             if (back < 0) break;
             cur = back;
@@ -149,9 +204,12 @@ __global__ void __launch_bounds__(kDpThreads) dp_kernel(const DpJob *__restrict_
 
 }  // namespace
 
-void launch_dp(const DpJob *d_jobs, int njobs, cudaStream_t s) {
+void launch_dp(const DpJob *d_jobs, int njobs, int64_t max_window, cudaStream_t s) {
     if (njobs <= 0) return;
-    dp_kernel<<<njobs, kDpThreads, 0, s>>>(d_jobs);
+    const int held = (int)std::min<int64_t>(max_window, kRowsHeld);
+    const size_t smem = 2 * (size_t)held * sizeof(double);
+    if (smem > 32 * 1024) cudaFuncSetAttribute(dp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    dp_kernel<<<njobs, kDpThreads, smem, s>>>(d_jobs, held);
     launch_counter() += 1;
 }
 

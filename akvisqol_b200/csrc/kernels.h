@@ -48,8 +48,8 @@ struct DpJob {
     const int64_t *lo, *hi;
     int32_t np;
     int64_t nf_deg;
-    double *dp;
-    int64_t *bt;
+    double *dp;   // np x nf_deg, rows too long for the kernel's shared memory
+    int32_t *bt;  // np x nf_deg
     int64_t *offset;  // np: matched offset, -1 when not reached
     uint8_t *valid;   // np
 };
@@ -215,6 +215,7 @@ void launch_stats(const StatsJob *d_jobs, int njobs, int nb, cudaStream_t s);
 void launch_fast_quotient(const double *num, const double *den, double *out, size_t count, cudaStream_t s);
 
 // k_dp.cu
-void launch_dp(const DpJob *d_jobs, int njobs, cudaStream_t s);
+// max_window: the largest hi - lo + 1 of the jobs' rows.
+void launch_dp(const DpJob *d_jobs, int njobs, int64_t max_window, cudaStream_t s);
 
 }  // namespace vqb

@@ -298,11 +298,14 @@ int visqol_b200_dp(const double *sims, size_t np, size_t nf_deg, const int64_t *
     return guarded([&] {
         vqb::Engine &e = stage_engine();
         DBuf<double> ds(sims, np * nf_deg), dpb(np * nf_deg);
-        DBuf<int64_t> dlo(lo, np), dhi(hi, np), bt(np * nf_deg), off(np);
+        DBuf<int64_t> dlo(lo, np), dhi(hi, np), off(np);
+        DBuf<int32_t> bt(np * nf_deg);
         DBuf<uint8_t> val(np);
         vqb::DpJob job{ds.p, dlo.p, dhi.p, (int32_t)np, (int64_t)nf_deg, dpb.p, bt.p, off.p, val.p};
         DBuf<vqb::DpJob> dj(&job, 1);
-        vqb::launch_dp(dj.p, 1, e.stream());
+        int64_t max_window = 0;
+        for (size_t p = 0; p < np; ++p) max_window = std::max(max_window, hi[p] - lo[p] + 1);
+        vqb::launch_dp(dj.p, 1, max_window, e.stream());
         VQB_CUDA(cudaStreamSynchronize(e.stream()));
         off.get(offset, np);
         val.get(valid, np);
