@@ -548,12 +548,13 @@ Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, con
     if (opt_.form == kFormExact) {
         // a rule's shape (VISQOL_TUNE_0 may fix another)
         const std::vector<int> shapes = gammatone_frames_shapes(nbi);
-        plan.tile = tuned(kTuneGammatone, opt_.form, nbi, {shapes[0]}, [](int) {}, stream_, &shapes);
+        plan.tile = tuned(kTuneGammatone, opt_.form, nbi, {gammatone_frames_per_cta(nbi, (int64_t)plan.frames)},
+                          [](int) {}, stream_, &shapes);
     } else {
         plan.tile = gammatone_staged_frames_per_cta();
     }
     plan.d_jobs = upload(jobs);
-    plan.d_tiles = upload_tiles(jobs, plan.tile, &plan.ntiles);
+    plan.d_tiles = upload_tiles(jobs, std::max(plan.tile, 1), &plan.ntiles);
     return plan;
 }
 
@@ -858,9 +859,9 @@ void Engine::spectrogram(const host::Filterbank &fb, const double *d_hann, size_
     SpecJob job{VSig{d_x, 0, (int64_t)len, (int64_t)len}, (int64_t)nf, d_out};
     const std::vector<SpecJob> jobs{job};
     const SpecJob *d_job = upload(jobs);
-    const int nbi = (int)fb.nb, F = gammatone_frames_per_cta(nbi);
+    const int nbi = (int)fb.nb, F = gammatone_frames_per_cta(nbi, (int64_t)nf);
     int ntiles = 0;
-    const void *d_tiles = upload_tiles(jobs, F, &ntiles);
+    const void *d_tiles = upload_tiles(jobs, std::max(F, 1), &ntiles);
     flush_uploads();
     launch_gammatone(d_job, d_tiles, ntiles, d_coeffs, nbi, d_hann, (int)window, (int)hop, F, stream_);
     sync();

@@ -151,7 +151,8 @@ void launch_lag32(const LagJob *d_jobs, int njobs, int64_t n, bool raw, const fl
 void launch_refine_approx(const LagJob *d_job, int64_t n, int nchunks, cudaStream_t s);
 
 // k_gammatone.cu
-int gammatone_frames_per_cta(int nb);
+constexpr int kGammatoneSplit = 0;  // tiles of one frame, a band over four lanes
+int gammatone_frames_per_cta(int nb, int64_t frames);
 std::vector<int> gammatone_frames_shapes(int nb);  // all valid frames per CTA, the rule's first
 size_t gammatone_tile_size();
 void fill_gammatone_tile(void *dst, int job, int frame0);
