@@ -25,6 +25,8 @@
 #include <tuple>
 #include <mutex>
 #include <functional>
+#include <atomic>
+#include <system_error>
 #include <future>
 
 #include "engine.h"
@@ -177,6 +179,9 @@ Engine::~Engine() {
     if (ev_piece_) cudaEventDestroy(ev_piece_);
     for (auto p : slot_) cudaFree(p);
     if (copy_) cudaStreamDestroy(copy_);
+    cudaFreeHost(piece_host_);
+    for (auto e : piece_done_)
+        if (e) cudaEventDestroy(e);
     if (ev_inputs_) cudaEventDestroy(ev_inputs_);
     if (ev_ref_done_) cudaEventDestroy(ev_ref_done_);
     if (side_) cudaStreamDestroy(side_);
@@ -323,6 +328,77 @@ void Engine::flush_uploads() {
     VQB_CUDA(cudaMemcpyAsync(up_dev_ + up_begin_, up_host_ + up_begin_, bytes, cudaMemcpyHostToDevice, stream_));
     timing_.h2d_bytes += bytes;
     up_begin_ = up_end_;
+}
+
+// The driver's own copy from pageable memory fills its staging buffers on
+// one thread. Four threads fill page-locked pieces of 512 KB, each with one in
+// flight while it fills the other: a minute's pair (46 MB) 4.1 to 2.1 ms, at
+// the link's 25 GB/s. Below 16 MB the driver's copy is as fast (7.7 MB 0.32
+// ms against 0.44); page-locked signals need no staging.
+void Engine::upload_signals(const std::vector<HostCopy> &copies) {
+    constexpr size_t kMinBytes = size_t(16) << 20;
+    std::vector<HostCopy> staged;
+    size_t bytes = 0;
+    for (const HostCopy &c : copies) {
+        if (!c.len) continue;
+        timing_.h2d_bytes += c.len * sizeof(double);
+        cudaPointerAttributes attr{};
+        const cudaError_t known = cudaPointerGetAttributes(&attr, c.src);
+        if (known != cudaSuccess) cudaGetLastError();
+        if (known == cudaSuccess && attr.type == cudaMemoryTypeUnregistered) {
+            staged.push_back(c);
+            bytes += c.len * sizeof(double);
+        } else {
+            VQB_CUDA(cudaMemcpyAsync(c.dst, c.src, c.len * sizeof(double), cudaMemcpyHostToDevice, stream_));
+        }
+    }
+    if (bytes < kMinBytes) {
+        for (const HostCopy &c : staged)
+            VQB_CUDA(cudaMemcpyAsync(c.dst, c.src, c.len * sizeof(double), cudaMemcpyHostToDevice, stream_));
+        return;
+    }
+    if (!piece_host_) {
+        for (auto &e : piece_done_)
+            if (!e) VQB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        VQB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&piece_host_), 2 * kCopyThreads * kCopyPiece, cudaHostAllocDefault));
+    }
+    struct Piece {
+        char *dst;
+        const char *src;
+        size_t bytes;
+    };
+    std::vector<Piece> pieces;
+    for (const HostCopy &c : staged)
+        for (size_t o = 0, n = c.len * sizeof(double); o < n; o += kCopyPiece)
+            pieces.push_back({reinterpret_cast<char *>(c.dst) + o, reinterpret_cast<const char *>(c.src) + o,
+                              std::min(kCopyPiece, n - o)});
+    std::atomic<size_t> next{0};
+    std::exception_ptr errs[kCopyThreads];
+    auto work = [&](size_t t) {
+        try {
+            VQB_CUDA(cudaSetDevice(device_));
+            size_t turn = 2 * t;
+            for (size_t k = next++; k < pieces.size(); k = next++, turn ^= 1) {
+                char *buf = piece_host_ + turn * kCopyPiece;
+                VQB_CUDA(cudaEventSynchronize(piece_done_[turn]));
+                std::memcpy(buf, pieces[k].src, pieces[k].bytes);
+                VQB_CUDA(cudaMemcpyAsync(pieces[k].dst, buf, pieces[k].bytes, cudaMemcpyHostToDevice, stream_));
+                VQB_CUDA(cudaEventRecord(piece_done_[turn], stream_));
+            }
+        } catch (...) {
+            errs[t] = std::current_exception();
+        }
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (size_t t = 1; t < kCopyThreads; ++t) threads.emplace_back(work, t);
+    } catch (const std::system_error &) {
+        // fewer threads than asked for: the others take their pieces
+    }
+    work(0);
+    for (auto &t : threads) t.join();
+    for (const auto &e : errs)
+        if (e) std::rethrow_exception(e);
 }
 
 void Engine::begin_batch() {
@@ -944,6 +1020,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     record(events_[0]);
 
     // ---- inputs -----------------------------------------------------------
+    std::vector<HostCopy> copies;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
         s.prep = prepared ? prepared[i] : nullptr;
@@ -962,20 +1039,18 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             s.deg = degs[i];
         } else {
             double *d = arena_.alloc_n<double>(s.dl);
-            if (s.dl) VQB_CUDA(cudaMemcpyAsync(d, degs[i], s.dl * sizeof(double), cudaMemcpyHostToDevice, stream_));
-            timing_.h2d_bytes += s.dl * sizeof(double);
+            copies.push_back({d, degs[i], s.dl});
             s.deg = d;
             if (s.prep) {
                 s.ref = s.prep->d_sig;
             } else {
                 double *r = arena_.alloc_n<double>(s.rl);
-                if (s.rl)
-                    VQB_CUDA(cudaMemcpyAsync(r, refs[i], s.rl * sizeof(double), cudaMemcpyHostToDevice, stream_));
-                timing_.h2d_bytes += s.rl * sizeof(double);
+                copies.push_back({r, refs[i], s.rl});
                 s.ref = r;
             }
         }
     }
+    upload_signals(copies);
 
     auto plan_prep_jobs = [&](const std::vector<PrepJob> &jobs) -> Launches {
         if (jobs.empty()) return {};

@@ -282,6 +282,17 @@ private:
     // the chunk small uploads gather in, and its range not yet sent
     char *up_host_ = nullptr, *up_dev_ = nullptr;
     size_t up_cap_ = 0, up_begin_ = 0, up_end_ = 0;
+    // Signals from host memory that is not page-locked go up through these
+    // page-locked pieces, two for each thread that fills them.
+    struct HostCopy {
+        double *dst;
+        const double *src;
+        size_t len;
+    };
+    void upload_signals(const std::vector<HostCopy> &copies);
+    static constexpr size_t kCopyThreads = 4, kCopyPiece = size_t(512) << 10;
+    char *piece_host_ = nullptr;  // 2 kCopyThreads pieces
+    cudaEvent_t piece_done_[2 * kCopyThreads] = {};
     std::map<uint32_t, RateCache> rates_;
     std::map<size_t, Twiddles> twiddles_;
     std::vector<cudaEvent_t> events_;
