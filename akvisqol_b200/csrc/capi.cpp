@@ -57,6 +57,7 @@ struct HostStaging {
     cudaStream_t copy = nullptr;
     cudaEvent_t piece = nullptr;
     std::vector<cudaEvent_t> chunk_done;
+    vqb::HostStager stager;
     ~HostStaging() {
         cudaSetDevice(device);
         if (copy) cudaStreamSynchronize(copy);
@@ -234,7 +235,8 @@ struct JoinAll {
 
 // Host-input batches through all lanes at once: the signals go up in chunks
 // of consecutive pairs, in order, on a copy stream of their own (one copy in
-// flight, so the lanes' own small uploads never queue behind a whole chunk),
+// flight, or a few staged pieces from pageable memory, so the lanes' own small
+// uploads never queue behind a whole chunk),
 // and the lanes take chunks from a shared queue as they free up, each
 // waiting on its chunk's upload. The GPU starts scoring when the first chunk
 // has landed, the transfer of the rest overlaps the scoring, and every chunk
@@ -308,7 +310,7 @@ bool run_lanes_queued(visqol_ctx *c, size_t n, const double *const *refs, const 
     // (host side) that the event they will wait on has been recorded
     std::mutex mu;
     std::condition_variable cv;
-    size_t recorded = 0;
+    std::vector<char> recorded(nk, 0);
     bool failed = false;
     std::exception_ptr upload_error;
     JoinAll uploader;
@@ -323,15 +325,34 @@ bool run_lanes_queued(visqol_ctx *c, size_t n, const double *const *refs, const 
                                          st.copy));
                 VQB_CUDA(cudaEventRecord(st.piece, st.copy));
             };
+            auto issued = [&](size_t k) {
+                VQB_CUDA(cudaEventRecord(st.chunk_done[k], st.copy));
+                std::lock_guard<std::mutex> lock(mu);
+                recorded[k] = 1;
+                cv.notify_all();
+            };
+            std::vector<vqb::HostStager::Copy> staged;
+            bool pageable = total >= vqb::HostStager::kMinBytes;
+            for (size_t k = 0; k < nk && pageable; ++k)
+                for (size_t i = bounds[k]; i < bounds[k + 1] && pageable; ++i) {
+                    auto add = [&](const double *dst, const double *src, size_t len) {
+                        if (!dst || !len) return;
+                        pageable = pageable && vqb::HostStager::pageable(src);
+                        staged.push_back({const_cast<double *>(dst), src, len, k});
+                    };
+                    add(d_ref[i], refs[i], ref_lens[i]);
+                    add(d_deg[i], degs[i], deg_lens[i]);
+                }
+            if (pageable) {
+                st.stager.run(device, st.copy, staged, nk, issued);
+                return;
+            }
             for (size_t k = 0; k < nk; ++k) {
                 for (size_t i = bounds[k]; i < bounds[k + 1]; ++i) {
                     if (d_ref[i]) copy(d_ref[i], refs[i], ref_lens[i]);
                     if (d_deg[i]) copy(d_deg[i], degs[i], deg_lens[i]);
                 }
-                VQB_CUDA(cudaEventRecord(st.chunk_done[k], st.copy));
-                std::lock_guard<std::mutex> lock(mu);
-                recorded = k + 1;
-                cv.notify_all();
+                issued(k);
             }
         } catch (...) {
             upload_error = std::current_exception();
@@ -351,8 +372,8 @@ bool run_lanes_queued(visqol_ctx *c, size_t n, const double *const *refs, const 
             std::vector<vqb::PairOutcome> part;
             {
                 std::unique_lock<std::mutex> lock(mu);
-                cv.wait(lock, [&] { return recorded > k || failed; });
-                if (recorded <= k) return false;
+                cv.wait(lock, [&] { return recorded[k] || failed; });
+                if (!recorded[k]) return false;
             }
             VQB_CUDA(cudaStreamWaitEvent(e.stream(), st.chunk_done[k], 0));
             const size_t b0 = bounds[k], m = bounds[k + 1] - b0;

@@ -179,9 +179,6 @@ Engine::~Engine() {
     if (ev_piece_) cudaEventDestroy(ev_piece_);
     for (auto p : slot_) cudaFree(p);
     if (copy_) cudaStreamDestroy(copy_);
-    cudaFreeHost(piece_host_);
-    for (auto e : piece_done_)
-        if (e) cudaEventDestroy(e);
     if (ev_inputs_) cudaEventDestroy(ev_inputs_);
     if (ev_ref_done_) cudaEventDestroy(ev_ref_done_);
     if (side_) cudaStreamDestroy(side_);
@@ -330,60 +327,60 @@ void Engine::flush_uploads() {
     up_begin_ = up_end_;
 }
 
+HostStager::~HostStager() {
+    cudaFreeHost(host_);
+    for (auto e : done_)
+        if (e) cudaEventDestroy(e);
+}
+
+bool HostStager::pageable(const void *p) {
+    cudaPointerAttributes attr{};
+    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return attr.type == cudaMemoryTypeUnregistered;
+}
+
 // The driver's own copy from pageable memory fills its staging buffers on
 // one thread. Four threads fill page-locked pieces of 512 KB, each with one in
 // flight while it fills the other: a minute's pair (46 MB) 4.1 to 2.1 ms, at
 // the link's 25 GB/s. Below 16 MB the driver's copy is as fast (7.7 MB 0.32
-// ms against 0.44); page-locked signals need no staging.
-void Engine::upload_signals(const std::vector<HostCopy> &copies) {
-    constexpr size_t kMinBytes = size_t(16) << 20;
-    std::vector<HostCopy> staged;
-    size_t bytes = 0;
-    for (const HostCopy &c : copies) {
-        if (!c.len) continue;
-        timing_.h2d_bytes += c.len * sizeof(double);
-        cudaPointerAttributes attr{};
-        const cudaError_t known = cudaPointerGetAttributes(&attr, c.src);
-        if (known != cudaSuccess) cudaGetLastError();
-        if (known == cudaSuccess && attr.type == cudaMemoryTypeUnregistered) {
-            staged.push_back(c);
-            bytes += c.len * sizeof(double);
-        } else {
-            VQB_CUDA(cudaMemcpyAsync(c.dst, c.src, c.len * sizeof(double), cudaMemcpyHostToDevice, stream_));
-        }
-    }
-    if (bytes < kMinBytes) {
-        for (const HostCopy &c : staged)
-            VQB_CUDA(cudaMemcpyAsync(c.dst, c.src, c.len * sizeof(double), cudaMemcpyHostToDevice, stream_));
-        return;
-    }
-    if (!piece_host_) {
-        for (auto &e : piece_done_)
+// ms against 0.44).
+void HostStager::run(int device, cudaStream_t stream, const std::vector<Copy> &copies, size_t groups,
+                     const std::function<void(size_t)> &issued) {
+    if (!host_) {
+        for (auto &e : done_)
             if (!e) VQB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        VQB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&piece_host_), 2 * kCopyThreads * kCopyPiece, cudaHostAllocDefault));
+        VQB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&host_), 2 * kThreads * kPiece, cudaHostAllocDefault));
     }
     struct Piece {
         char *dst;
         const char *src;
-        size_t bytes;
+        size_t bytes, group;
     };
     std::vector<Piece> pieces;
-    for (const HostCopy &c : staged)
-        for (size_t o = 0, n = c.len * sizeof(double); o < n; o += kCopyPiece)
+    std::vector<std::atomic<size_t>> left(groups);
+    for (auto &l : left) l = 0;
+    for (const Copy &c : copies)
+        for (size_t o = 0, n = c.len * sizeof(double); o < n; o += kPiece, ++left[c.group])
             pieces.push_back({reinterpret_cast<char *>(c.dst) + o, reinterpret_cast<const char *>(c.src) + o,
-                              std::min(kCopyPiece, n - o)});
+                              std::min(kPiece, n - o), c.group});
+    for (size_t g = 0; g < groups; ++g)
+        if (left[g] == 0 && issued) issued(g);
     std::atomic<size_t> next{0};
-    std::exception_ptr errs[kCopyThreads];
+    std::exception_ptr errs[kThreads];
     auto work = [&](size_t t) {
         try {
-            VQB_CUDA(cudaSetDevice(device_));
+            VQB_CUDA(cudaSetDevice(device));
             size_t turn = 2 * t;
             for (size_t k = next++; k < pieces.size(); k = next++, turn ^= 1) {
-                char *buf = piece_host_ + turn * kCopyPiece;
-                VQB_CUDA(cudaEventSynchronize(piece_done_[turn]));
-                std::memcpy(buf, pieces[k].src, pieces[k].bytes);
-                VQB_CUDA(cudaMemcpyAsync(pieces[k].dst, buf, pieces[k].bytes, cudaMemcpyHostToDevice, stream_));
-                VQB_CUDA(cudaEventRecord(piece_done_[turn], stream_));
+                const Piece &p = pieces[k];
+                VQB_CUDA(cudaEventSynchronize(done_[turn]));
+                std::memcpy(host_ + turn * kPiece, p.src, p.bytes);
+                VQB_CUDA(cudaMemcpyAsync(p.dst, host_ + turn * kPiece, p.bytes, cudaMemcpyHostToDevice, stream));
+                VQB_CUDA(cudaEventRecord(done_[turn], stream));
+                if (--left[p.group] == 0 && issued) issued(p.group);
             }
         } catch (...) {
             errs[t] = std::current_exception();
@@ -391,7 +388,7 @@ void Engine::upload_signals(const std::vector<HostCopy> &copies) {
     };
     std::vector<std::thread> threads;
     try {
-        for (size_t t = 1; t < kCopyThreads; ++t) threads.emplace_back(work, t);
+        for (size_t t = 1; t < kThreads; ++t) threads.emplace_back(work, t);
     } catch (const std::system_error &) {
         // fewer threads than asked for: the others take their pieces
     }
@@ -399,6 +396,29 @@ void Engine::upload_signals(const std::vector<HostCopy> &copies) {
     for (auto &t : threads) t.join();
     for (const auto &e : errs)
         if (e) std::rethrow_exception(e);
+}
+
+// (page-locked signals need no staging)
+void Engine::upload_signals(const std::vector<HostStager::Copy> &copies) {
+    std::vector<HostStager::Copy> staged;
+    size_t bytes = 0;
+    auto direct = [&](const HostStager::Copy &c) {
+        VQB_CUDA(cudaMemcpyAsync(c.dst, c.src, c.len * sizeof(double), cudaMemcpyHostToDevice, stream_));
+    };
+    for (const HostStager::Copy &c : copies) {
+        if (!c.len) continue;
+        timing_.h2d_bytes += c.len * sizeof(double);
+        if (HostStager::pageable(c.src)) {
+            staged.push_back(c);
+            bytes += c.len * sizeof(double);
+        } else {
+            direct(c);
+        }
+    }
+    if (bytes < HostStager::kMinBytes)
+        for (const HostStager::Copy &c : staged) direct(c);
+    else
+        stager_.run(device_, stream_, staged, 1, nullptr);
 }
 
 void Engine::begin_batch() {
@@ -1020,7 +1040,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     record(events_[0]);
 
     // ---- inputs -----------------------------------------------------------
-    std::vector<HostCopy> copies;
+    std::vector<HostStager::Copy> copies;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
         s.prep = prepared ? prepared[i] : nullptr;
@@ -1039,13 +1059,13 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             s.deg = degs[i];
         } else {
             double *d = arena_.alloc_n<double>(s.dl);
-            copies.push_back({d, degs[i], s.dl});
+            copies.push_back({d, degs[i], s.dl, 0});
             s.deg = d;
             if (s.prep) {
                 s.ref = s.prep->d_sig;
             } else {
                 double *r = arena_.alloc_n<double>(s.rl);
-                copies.push_back({r, refs[i], s.rl});
+                copies.push_back({r, refs[i], s.rl, 0});
                 s.ref = r;
             }
         }

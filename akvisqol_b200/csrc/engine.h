@@ -128,6 +128,33 @@ struct PreparedRef {
     ~PreparedRef();
 };
 
+// Uploads from pageable host memory: several threads fill page-locked pieces,
+// two each, and send them on one stream.
+class HostStager {
+  public:
+    struct Copy {
+        double *dst;
+        const double *src;
+        size_t len;
+        size_t group;
+    };
+    HostStager() = default;
+    HostStager(const HostStager &) = delete;
+    HostStager &operator=(const HostStager &) = delete;
+    ~HostStager();  // (the stream has been synchronized)
+    static bool pageable(const void *p);
+    // issued(g): every copy of group g is on the stream; called once a group,
+    // from any of the threads. Returns when all are issued.
+    void run(int device, cudaStream_t stream, const std::vector<Copy> &copies, size_t groups,
+             const std::function<void(size_t)> &issued);
+    static constexpr size_t kMinBytes = size_t(16) << 20;
+
+  private:
+    static constexpr size_t kThreads = 4, kPiece = size_t(512) << 10;
+    char *host_ = nullptr;  // 2 kThreads pieces
+    cudaEvent_t done_[2 * kThreads] = {};
+};
+
 class Engine {
 public:
     Engine(int device, const Options &opt, std::shared_ptr<const host::Svr> svr,
@@ -282,17 +309,8 @@ private:
     // the chunk small uploads gather in, and its range not yet sent
     char *up_host_ = nullptr, *up_dev_ = nullptr;
     size_t up_cap_ = 0, up_begin_ = 0, up_end_ = 0;
-    // Signals from host memory that is not page-locked go up through these
-    // page-locked pieces, two for each thread that fills them.
-    struct HostCopy {
-        double *dst;
-        const double *src;
-        size_t len;
-    };
-    void upload_signals(const std::vector<HostCopy> &copies);
-    static constexpr size_t kCopyThreads = 4, kCopyPiece = size_t(512) << 10;
-    char *piece_host_ = nullptr;  // 2 kCopyThreads pieces
-    cudaEvent_t piece_done_[2 * kCopyThreads] = {};
+    HostStager stager_;
+    void upload_signals(const std::vector<HostStager::Copy> &copies);
     std::map<uint32_t, RateCache> rates_;
     std::map<size_t, Twiddles> twiddles_;
     std::vector<cudaEvent_t> events_;
