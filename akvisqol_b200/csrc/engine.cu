@@ -127,7 +127,12 @@ void *PinnedArena::alloc(size_t bytes) {
         }
         ++current_;
     }
-    Chunk c{nullptr, std::max(bytes, size_t(64) << 20), 0};
+    // Page-locking costs ~0.6 ms a megabyte, on an engine's first batch: a
+    // small chunk, then as much again as there is. (64 MB at once took 26 to
+    // 37 ms: a fresh exact context's first pair 58 ms, now 25.)
+    size_t held = 0;
+    for (const Chunk &h : chunks_) held += h.size;
+    Chunk c{nullptr, std::max({bytes, held, size_t(2) << 20}), 0};
     VQB_CUDA(cudaMallocHost(&c.base, c.size));
     c.used = bytes;
     chunks_.push_back(c);
@@ -188,7 +193,6 @@ Engine::~Engine() {
         cudaFree(kv.second.d_hann);
         cudaFree(kv.second.d_spectral);
     }
-    for (auto &kv : twiddles_) cudaFree(const_cast<double2 *>(kv.second.top));
     for (auto e : events_) cudaEventDestroy(e);
     for (auto e : gt_events_)
         if (e) cudaEventDestroy(e);
@@ -261,9 +265,33 @@ const Engine::RateCache &Engine::rate_cache(uint32_t sr) {
     return rates_.emplace(sr, std::move(rc)).first->second;
 }
 
-Engine::Twiddles Engine::twiddles(size_t n) {
+// A size's tables on a device, for as long as an engine there holds them:
+// formed once for all lanes (2^20 points: ~25 ms of sines and 24 MB, which
+// every lane of every mode would pay and keep for itself).
+struct Engine::TwiddleTable {
+    int device;
+    double2 *base;
+    Twiddles view;
+    TwiddleTable(int dev, double2 *d, const Twiddles &v) : device(dev), base(d), view(v) {}
+    TwiddleTable(const TwiddleTable &) = delete;
+    TwiddleTable &operator=(const TwiddleTable &) = delete;
+    ~TwiddleTable() {
+        int cur = 0;
+        cudaGetDevice(&cur);
+        cudaSetDevice(device);
+        cudaFree(base);
+        cudaSetDevice(cur);
+    }
+};
+
+const Engine::Twiddles &Engine::twiddles(size_t n) {
     auto it = twiddles_.find(n);
-    if (it != twiddles_.end()) return it->second;
+    if (it != twiddles_.end()) return it->second->view;
+    static std::mutex mu;
+    static std::map<std::pair<int, size_t>, std::weak_ptr<const TwiddleTable>> shared;
+    std::lock_guard<std::mutex> lock(mu);
+    std::weak_ptr<const TwiddleTable> &entry = shared[{device_, n}];
+    if (auto held = entry.lock()) return (twiddles_[n] = std::move(held))->view;
     // top[k] = W_n^k (k < n/2), then the block passes' W_B^k = top[k * n/B].
     // then the fused lag search's stage-major column twiddles.
     std::vector<double2> t = host::twiddles(n);
@@ -291,9 +319,11 @@ Engine::Twiddles Engine::twiddles(size_t n) {
         VQB_CUDA(cudaMemcpyAsync(d32, t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice, stream_));
         VQB_CUDA(cudaStreamSynchronize(stream_));
     }
-    Twiddles tw{d, d + half, d + cols_at, d + stages_at, d32, d32 + (cols_at - half), d32 + (stages_at - half)};
-    twiddles_[n] = tw;
-    return tw;
+    // (on the device before another engine's streams see it)
+    const Twiddles tw{d, d + half, d + cols_at, d + stages_at, d32, d32 + (cols_at - half), d32 + (stages_at - half)};
+    auto made = std::make_shared<const TwiddleTable>(device_, d, tw);
+    entry = made;
+    return (twiddles_[n] = std::move(made))->view;
 }
 
 template <class T>

@@ -219,7 +219,8 @@ public:
         const double2 *top, *block, *cols, *stages;
         const float2 *block32, *cols32, *stages32;  // the same tables rounded to f32 (the f32 search)
     };
-    Twiddles twiddles(size_t n);
+    struct TwiddleTable;
+    const Twiddles &twiddles(size_t n);
 
 private:
     struct RateCache {
@@ -312,7 +313,7 @@ private:
     HostStager stager_;
     void upload_signals(const std::vector<HostStager::Copy> &copies);
     std::map<uint32_t, RateCache> rates_;
-    std::map<size_t, Twiddles> twiddles_;
+    std::map<size_t, std::shared_ptr<const TwiddleTable>> twiddles_;  // (shared by the device's engines)
     std::vector<cudaEvent_t> events_;
     cudaStream_t side_ = nullptr;    // reference spectrograms, concurrent with the lag phase
     cudaEvent_t ev_inputs_ = nullptr, ev_ref_done_ = nullptr;
