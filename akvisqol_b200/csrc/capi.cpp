@@ -441,12 +441,15 @@ void run_lanes(visqol_ctx *c, size_t n, const double *const *refs, const size_t 
     // pairs as they free up, each lane's first chunk at 30% of the average,
     // so that the lanes fall out of step and their light phases (host
     // planning, small kernels) overlap other lanes' heavy ones instead of
-    // coinciding. Measured on one B200 (128 pairs of 10 s): three chunks a
-    // lane score the FP32 and FP64-FMA forms ~1% faster than one share a
-    // lane; the exact form, whose lanes wait on serial sums, 6-17% slower
-    // with chunks, so it keeps one share a lane. VISQOL_DEVICE_CHUNKS
-    // overrides (chunks a lane, 0: one share a lane).
-    size_t dev_chunks = c->opt.form == vqb::kFormExact ? 0 : 3;
+    // coinciding. One chunk a lane below 32 pairs a lane: smaller chunks are
+    // more launches of less work (64 fast 10 s pairs 10.3 ms, with three
+    // chunks a lane 10.7; 20 speech pairs 1.6, with three 2.7). From there on
+    // three chunks a lane are 1-3% faster (256 fast pairs 39.5 ms against
+    // 40.1, 300 speech pairs 17.6 against 17.8). The exact form keeps one
+    // share a lane, dealt longest first (64 pairs of 10 s 24.3 ms, with three
+    // chunks 25.1). VISQOL_DEVICE_CHUNKS overrides (chunks a lane, 0: one
+    // share a lane).
+    size_t dev_chunks = c->opt.form == vqb::kFormExact ? 0 : n >= 32 * L ? 3 : 1;
     if (const char *env = std::getenv("VISQOL_DEVICE_CHUNKS"))
         dev_chunks = std::min<size_t>(16, (size_t)std::strtoull(env, nullptr, 10));
     if (device_inputs && !grads && dev_chunks > 0 && n >= dev_chunks * L) {
