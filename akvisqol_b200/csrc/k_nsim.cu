@@ -426,6 +426,8 @@ void launch_table(const TableTask *d_tasks, int ntasks, int max_offsets, int nb,
         // distances; 3.06 to 2.64 ms of a batch of 32 exact audio pairs)
         if (fast && P == 30)
             table_kernel<true, 30><<<grid, threads, smem, s>>>(t, nb, P);
+        else if (fast && P == 20)
+            table_kernel<true, 20><<<grid, threads, smem, s>>>(t, nb, P);
         else if (fast)
             table_kernel<true, 0><<<grid, threads, smem, s>>>(t, nb, P);
         else if (P == 30)
