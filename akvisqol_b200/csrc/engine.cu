@@ -612,20 +612,15 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
     const size_t np = nfr / std::max<size_t>(1, P) + 1;
     const size_t n_global = host::fft_size_for(std::max(rl, dl));
     const size_t n_slice = host::fft_size_for(2 * P * H + 2);
-    // FMA forms: a frame's spectrum and partial sums (k_spectral.cu), up to 2048
-    // frames of 4096 points; the degraded and realigned spectrograms share theirs
-    const size_t points = host::fft_size_for(host::analysis_geometry(sample_rate).window);
-    auto spectral_frames = [&](size_t nf) { return std::min<size_t>(nf + 63, (size_t(1) << 24) / points); };
-    const size_t spectral = 6 * points * (spectral_frames(nfr) + spectral_frames(std::max(nfd, 2 * np * (P + 2))));
-    const size_t sums = 2 * serial_sum_scratch(2, (int64_t)std::max(rl, dl)) +
-                        serial_sum_scratch((int)(2 * np), (int64_t)(2 * P * H + 2));
     size_t b = 8 * (rl + dl)                                   // inputs
-               + std::max(sums, spectral)                      // exact form's sums, FMA forms' spectra
                + 16 * n_global + 16 * 1024                     // lag search and argmax parts
                + 8 * al                                        // aligned, scaled degraded signal
                + 8 * NB * (2 * nfr + 2 * nfd + 4 * width)      // spectrograms, prepared copies, plane
-               + np * (8 * 3 * NB * P + 24 * nfd + 8 * (3 * NB + 1) + 16)  // terms, table, DP, stats
+               + np * (8 * 4 * NB * P + 24 * nfd + 8 * (3 * NB + 1) + 16)  // terms, table, DP, stats
                + np * (16 * n_slice + 8 * 4 * NB * (2 * P + 2) + 256);     // realignment slices
+    // The lag searches nominate in f32, 8 bytes a point; the other 8 hold an
+    // exact rerun, or leave room for the exact form's sums and the FMA forms'
+    // spectra (44 KB a frame for up to 2048 frames, once for a batch).
     b += b / 4 + (size_t(1) << 20);  // job tables, tiles, rounding slack
     return b;
 }
@@ -644,7 +639,7 @@ const void *Engine::upload_tiles(const std::vector<SpecJob> &jobs, int F, int *n
 }
 
 Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc,
-                                           const SpecPlan *before) {
+                                           const SpecPlan *before, size_t room) {
     SpecPlan plan;
     plan.rc = &rc;
     for (const SpecJob &j : jobs) plan.frames += (size_t)j.nf;
@@ -665,10 +660,13 @@ Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, con
                 frames[k++] = SpectralFrame{j.sig.base + first, j.out + f, (int32_t)lo, (int32_t)hi, j.nf};
             }
         plan.d_frames = upload(frames);
-        plan.scratch_count = spectral_scratch_count(*rc.spectral, (int)plan.frames);
-        plan.scratch = before && before->scratch_count >= plan.scratch_count
-                           ? before->scratch
-                           : arena_.alloc_n<double>(plan.scratch_count);
+        plan.scratch_count = spectral_scratch_count(*rc.spectral, (int)std::max(plan.frames, room));
+        if (before && before->scratch_count >= spectral_scratch_count(*rc.spectral, (int)plan.frames)) {
+            plan.scratch = before->scratch;
+            plan.scratch_count = before->scratch_count;
+        } else {
+            plan.scratch = arena_.alloc_n<double>(plan.scratch_count);
+        }
         return plan;
     }
     if (opt_.form == kFormExact) {
@@ -1124,6 +1122,8 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     // Reference spectrograms need only the reference signal: they run on a
     // side stream while the main stream does the lag-phase work.
     std::vector<SpecJob> ref_jobs;
+    SpecPlan ref_spec;
+    size_t deg_frames = 0;  // about what the degraded spectrograms take
     std::vector<VadJob> vads;
     std::vector<size_t> vad_at(n, SIZE_MAX);
     size_t nloud = 0, nlag = 0;
@@ -1140,6 +1140,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         }
         const VSig sig{s.ref, 0, (int64_t)s.rl, (int64_t)s.rl};
         s.nf_ref = host::num_frames(s.rl, W, H);
+        deg_frames += std::max(s.nf_ref, host::num_frames(s.dl, W, H)) + 16;
         s.ref_raw = arena_.alloc_n<double>(NB * s.nf_ref);
         ref_jobs.push_back(SpecJob{sig, (int64_t)s.nf_ref, s.ref_raw});
         if (opt_.speech) {
@@ -1211,7 +1212,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         std::vector<size_t> all(n);
         for (size_t i = 0; i < n; ++i) all[i] = i;
         // every upload of the phase goes up with the first flush
-        const SpecPlan ref_spec = plan_spectrograms(ref_jobs, rc);
+        ref_spec = plan_spectrograms(ref_jobs, rc, nullptr, deg_frames);
         const Launches do_sums = plan_sums(sums), do_lags = plan_lag_jobs(lag_jobs, false, d_lstat),
                        do_aligned = plan_aligned(all), do_vad = plan_vad(vads);
         run_gammatone(ref_spec, side_);
@@ -1365,7 +1366,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
 
     // ---- 3: spectrograms, prep, NSIM table, DP, match statistics ----------
     // every upload of the phase goes up with the first flush
-    const SpecPlan deg_spec = plan_spectrograms(spec_jobs, rc);
+    const SpecPlan deg_spec = plan_spectrograms(spec_jobs, rc, &ref_spec);
     const Launches do_prep = plan_prep_jobs(prep_jobs);
     const void *d_scale = upload_bytes(scale_args.data(), scale_args.size());
     const PlaneJob *d_planes = upload(plane_jobs);
@@ -1376,6 +1377,9 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     const TableTask *d_table = upload(table_rows);
     flush_uploads();
     if (nscale) launch_scale(d_scale, nscale, max_al, stream_);
+    // the reference spectrograms' scratch is used again, and what follows
+    // reads their results
+    if (deg_spec.scratch && deg_spec.scratch == ref_spec.scratch) VQB_CUDA(cudaStreamWaitEvent(stream_, ev_ref_done_, 0));
     record(events_[2]);
     run_gammatone(deg_spec, stream_);
     record(events_[3]);

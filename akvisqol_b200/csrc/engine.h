@@ -266,8 +266,10 @@ private:
         const void *d_tiles = nullptr;
         int ntiles = 0, tile = 0;
     };
-    // before: a plan run earlier on the same stream, whose scratch may be used again
-    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, const SpecPlan *before = nullptr);
+    // before: a plan whose launches come before this one's, whose scratch is
+    // used again if it is large enough; room: frames to make the scratch large enough for
+    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, const SpecPlan *before = nullptr,
+                               size_t room = 0);
     void run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin = nullptr,
                           cudaEvent_t end = nullptr);
     const void *upload_tiles(const std::vector<SpecJob> &jobs, int F, int *ntiles);
