@@ -9,8 +9,8 @@ copy); ``e2e`` times the public call with pinned host buffers, host-to-device
 copies and result read-back included. Each step's inputs (~0.5 GB) exceed
 the 126 MB L2, so no flush is needed between steps.
 
-The headline form is --precision (fast: f32 gammatone stages; balanced:
-f64 with FMA; exact: the CPU path's f64 operation order); the other forms
+The headline form is --precision (fast and balanced: f64 with FMA, gammatone
+energies from power spectra; exact: the CPU path's f64 operation order); the other forms
 are timed the same way and reported under "forms", each with its largest
 |dMOS| against the CPU model on the baseline sample.
 
@@ -44,15 +44,16 @@ METRICS = {
     "balanced": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), FP64 FMA form, 1 B200",
     "exact": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), exact FP64 form, 1 B200",
 }
-DTYPES = {"fast": "f32 (gammatone stages 3-4 above the lowest band group, lag-search transform; rescoring, "
-                  "NSIM, DP, MOS in f64)",
+DTYPES = {"fast": "f64 (FMA); the lag search's nominating transform in f32, its rescoring in f64",
           "balanced": "f64 (FMA); the lag search's nominating transform in f32, its rescoring in f64",
           "exact": "f64; the lag search's nominating transform in f32, its rescoring in f64"}
-# gammatone: pipe-peak kind of visqol_b200_peak and the algorithm's flops per
-# sample, the same for every form: 4 biquads of 7 flops, the window multiply
-# and the square-accumulate (reference src/gammatone.zig:268-306)
-ROOF = {"exact": (0, 31.0, "fp64-pipe (mul/add)"), "balanced": (1, 31.0, "fp64-pipe (fma)"),
-        "fast": (2, 31.0, "fp32-pipe (fma), stages 1-2 on the fp64 pipe")}
+# gammatone: pipe-peak kind of visqol_b200_peak and the flops per sample and
+# band that the form's algorithm takes. Exact: 4 biquads of 7, the window
+# multiply and the square-accumulate (reference src/gammatone.zig:268-306).
+# Power spectra (48 kHz): 185 k multiply-adds a frame for the transform, 131 k
+# for the band sums and 420 k for the tails, over 32 bands x 3840 samples.
+ROOF = {"exact": (0, 31.0, "fp64-pipe (mul/add)"), "balanced": (1, 12.0, "fp64-pipe (fma)"),
+        "fast": (1, 12.0, "fp64-pipe (fma)")}
 WORKLOAD = "audio-mode pairs, 10 s at 48 kHz (480,000 samples; degraded 481,776), seeded synthetic music-like generator"
 # HBM copy bandwidth of this pool's B200s when the driver's measurement
 # (MEASURED_PEAKS.json) is absent
