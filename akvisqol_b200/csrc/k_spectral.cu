@@ -26,16 +26,16 @@
 // transform ~185 k, the band sums 131 k, the tails 420 k: 0.74 M, where the
 // recurrence takes 14 a sample and band, 1.72 M. The two contractions run on
 // the f64 tensor instruction (mma m8n8k4: the FP64 pipe's full rate, one
-// instruction for 256 multiply-adds), and 32 frames are 28 independent pieces
+// instruction for 256 multiply-adds), and 32 frames are 42 independent pieces
 // of work instead of 32 recurrences of 3840 steps each. Measured per 48 kHz
-// frame in a launch of 2048: 27 ns for the spectrum, 47 for the band sums and
-// tails (36 at the FP64 pipe's rate), 4 to finish; the recurrence took 128 in
+// frame in a launch of 2048: 28 ns for the spectrum, 43 for the band sums and
+// tails (31 at the FP64 tensor rate), 5 to finish; the recurrence took 128 in
 // f64 and 105 with its last two stages in f32. A single 6.4 s pair's call went
 // from 1.34 ms to 0.70, 64 pairs of 10 s from 18.0 ms to 11.2.
 //
 // Three launches over up to 2048 48 kHz frames (a spectrum row is 33 KB; 2048
 // rows stay in the L2): spectrum_kernel, a CTA per frame; energy_kernel, a warp per
-// piece and tile of 32 or 64 frames; finish_kernel, the pieces added in order.
+// piece and tile of 32 frames; finish_kernel, the pieces added in order.
 // Every frame's values are formed in the same order whatever its batch.
 #include <algorithm>
 
