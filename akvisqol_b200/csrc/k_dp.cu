@@ -208,7 +208,10 @@ void launch_dp(const DpJob *d_jobs, int njobs, int64_t max_window, cudaStream_t 
     if (njobs <= 0) return;
     const int held = (int)std::min<int64_t>(max_window, kRowsHeld);
     const size_t smem = 2 * (size_t)held * sizeof(double);
-    if (smem > 32 * 1024) cudaFuncSetAttribute(dp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the same value from every thread: a smaller one would fail another's launch)
+    if (smem > 32 * 1024)
+        cudaFuncSetAttribute(dp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             2 * kRowsHeld * (int)sizeof(double));
     dp_kernel<<<njobs, kDpThreads, smem, s>>>(d_jobs, held);
     launch_counter() += 1;
 }

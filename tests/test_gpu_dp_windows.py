@@ -26,3 +26,32 @@ def test_windows(native, oracle, frames, rows, radius, ties):
     woff, wvalid, wreached = oracle.dp_backtrack(sims, lo, hi)
     assert reached == wreached
     assert np.array_equal(off, woff) and np.array_equal(valid, wvalid)
+
+
+def test_sizes_in_threads(native, oracle):
+    """Rows of different lengths launched by two threads at once: neither's
+    shared memory is taken back by the other."""
+    import functools
+    import threading
+    rng = np.random.default_rng(2)
+    jobs = []
+    for run, frames in ((native.dp, 2300), (functools.partial(native.dp, static_scratch=True), 12000)):
+        sims = rng.uniform(0, 1, (4, frames))
+        lo, hi = np.zeros(4, np.int64), np.full(4, frames - 1)
+        jobs.append((run, sims, lo, hi, oracle.dp_backtrack(sims, lo, hi)[0]))
+    wrong = []
+
+    def work(run, sims, lo, hi, want):
+        for _ in range(150):
+            try:
+                if not np.array_equal(run(sims, lo, hi)[0], want):
+                    wrong.append("offsets")
+            except Exception as e:  # noqa: BLE001
+                wrong.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:3]
