@@ -26,7 +26,6 @@
 #include <mutex>
 #include <functional>
 #include <atomic>
-#include <system_error>
 #include <future>
 
 #include "engine.h"
@@ -37,6 +36,7 @@
 
 #include "grad_host.h"
 #include "kernels.h"
+#include "threads.h"
 
 namespace vqb {
 
@@ -399,33 +399,18 @@ void HostStager::run(int device, cudaStream_t stream, const std::vector<Copy> &c
     for (size_t g = 0; g < groups; ++g)
         if (left[g] == 0 && issued) issued(g);
     std::atomic<size_t> next{0};
-    std::exception_ptr errs[kThreads];
-    auto work = [&](size_t t) {
-        try {
-            VQB_CUDA(cudaSetDevice(device));
-            size_t turn = 2 * t;
-            for (size_t k = next++; k < pieces.size(); k = next++, turn ^= 1) {
-                const Piece &p = pieces[k];
-                VQB_CUDA(cudaEventSynchronize(done_[turn]));
-                std::memcpy(host_ + turn * kPiece, p.src, p.bytes);
-                VQB_CUDA(cudaMemcpyAsync(p.dst, host_ + turn * kPiece, p.bytes, cudaMemcpyHostToDevice, stream));
-                VQB_CUDA(cudaEventRecord(done_[turn], stream));
-                if (--left[p.group] == 0 && issued) issued(p.group);
-            }
-        } catch (...) {
-            errs[t] = std::current_exception();
+    run_threads(kThreads, [&](size_t t) {
+        VQB_CUDA(cudaSetDevice(device));
+        size_t turn = 2 * t;
+        for (size_t k = next++; k < pieces.size(); k = next++, turn ^= 1) {
+            const Piece &p = pieces[k];
+            VQB_CUDA(cudaEventSynchronize(done_[turn]));
+            std::memcpy(host_ + turn * kPiece, p.src, p.bytes);
+            VQB_CUDA(cudaMemcpyAsync(p.dst, host_ + turn * kPiece, p.bytes, cudaMemcpyHostToDevice, stream));
+            VQB_CUDA(cudaEventRecord(done_[turn], stream));
+            if (--left[p.group] == 0 && issued) issued(p.group);
         }
-    };
-    std::vector<std::thread> threads;
-    try {
-        for (size_t t = 1; t < kThreads; ++t) threads.emplace_back(work, t);
-    } catch (const std::system_error &) {
-        // fewer threads than asked for: the others take their pieces
-    }
-    work(0);
-    for (auto &t : threads) t.join();
-    for (const auto &e : errs)
-        if (e) std::rethrow_exception(e);
+    });
 }
 
 // (page-locked signals need no staging)
@@ -1612,16 +1597,10 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     // The lattice mapping runs a few milliseconds of host interpreter per
     // pair: spread it over host threads (results are per pair).
     const size_t workers = lattice_ ? std::min<size_t>(n, std::max(1u, std::thread::hardware_concurrency() / 2)) : 1;
-    if (workers > 1) {
-        std::vector<std::thread> pool;
-        for (size_t w = 0; w < workers; ++w)
-            pool.emplace_back([&, w] {
-                for (size_t i = w; i < n; i += workers) finish(i);
-            });
-        for (auto &t : pool) t.join();
-    } else {
-        for (size_t i = 0; i < n; ++i) finish(i);
-    }
+    std::atomic<size_t> turn{0};
+    run_threads(workers, [&](size_t) {
+        for (size_t i = turn++; i < n; i = turn++) finish(i);
+    });
     if (grads) {
         for (size_t i = 0; i < n; ++i)
             if (ps[i].live && out[i].code == 0) ps[i].grad_ok = true;

@@ -5,10 +5,13 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <map>
 #include <mutex>
 #include <thread>
+
+#include "threads.h"
 
 namespace vqb {
 
@@ -204,15 +207,10 @@ std::shared_ptr<const SpectralTables> build(const std::vector<BandCoeffs> &run, 
     }
     cosines[N / 4] = cosines[3 * N / 4] = 0;
     std::vector<Band> bands(run.size());
-    {
-        std::vector<std::thread> pool;
-        const size_t workers = std::max<size_t>(1, std::min<size_t>(8, std::thread::hardware_concurrency()));
-        for (size_t w = 0; w < workers; ++w)
-            pool.emplace_back([&, w] {
-                for (size_t b = w; b < run.size(); b += workers) bands[b] = band_tables(run[b], window, N, cosines);
-            });
-        for (auto &th : pool) th.join();
-    }
+    std::atomic<size_t> next{0};
+    run_threads(std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency())), [&](size_t) {
+        for (size_t b = next++; b < run.size(); b = next++) bands[b] = band_tables(run[b], window, N, cosines);
+    });
     t->hann.assign((size_t)t->padded, 0.0);
     {
         const double denom = std::max(1.0, (double)window - 1.0);
