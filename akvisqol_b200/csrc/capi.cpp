@@ -199,6 +199,7 @@ void add_batch_timing(vqb::Timing &a, const vqb::Timing &x) {
     a.lag_kernel_ms += x.lag_kernel_ms;
     a.lag_bytes += x.lag_bytes;
     a.lag_reruns += x.lag_reruns;
+    a.arena_bytes = std::max(a.arena_bytes, x.arena_bytes);
 }
 
 // Lanes side by side: spans are the longest lane's, work counts add up.
@@ -220,6 +221,7 @@ void merge_lane_timing(vqb::Timing &t, const vqb::Timing &x) {
     t.lag_kernel_ms = std::max(t.lag_kernel_ms, x.lag_kernel_ms);
     t.lag_bytes += x.lag_bytes;
     t.lag_reruns += x.lag_reruns;
+    t.arena_bytes = std::max(t.arena_bytes, x.arena_bytes);
 }
 
 // Joins the threads it holds when it goes out of scope, so that an exception
@@ -955,6 +957,12 @@ int visqol_b200_last_timing(visqol_ctx *c, visqol_b200_timing *out) {
     out->lag_kernel_ms = t.lag_kernel_ms;
     out->lag_bytes = t.lag_bytes;
     out->lag_reruns = t.lag_reruns;
+    return VISQOL_OK;
+}
+
+int visqol_b200_last_batch_bytes(visqol_ctx *c, uint64_t *bytes) {
+    if (!c || !bytes) return fail(VISQOL_E_INVALID_ARGUMENT, "NULL argument");
+    *bytes = c->timing.arena_bytes;
     return VISQOL_OK;
 }
 

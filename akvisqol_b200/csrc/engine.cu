@@ -78,10 +78,12 @@ Arena::~Arena() {
 }
 void Arena::reset() {
     for (auto &c : chunks_) c.used = 0;
-    current_ = 0;
+    current_ = in_use_ = peak_ = 0;
 }
 void *Arena::alloc(size_t bytes) {
     bytes = round_up(bytes ? bytes : 1);
+    in_use_ += bytes;
+    peak_ = std::max(peak_, in_use_);
     while (current_ < chunks_.size()) {
         Chunk &c = chunks_[current_];
         if (c.used + bytes <= c.size) {
@@ -97,6 +99,12 @@ void *Arena::alloc(size_t bytes) {
     chunks_.push_back(c);
     current_ = chunks_.size() - 1;
     return c.base;
+}
+Arena::Mark Arena::mark() const { return {current_, current_ < chunks_.size() ? chunks_[current_].used : 0, in_use_}; }
+void Arena::rewind(const Mark &m) {
+    for (size_t i = m.chunk; i < chunks_.size(); ++i) chunks_[i].used = i == m.chunk ? m.used : 0;
+    current_ = m.chunk;
+    in_use_ = m.in_use;
 }
 void Arena::release() {
     for (auto &c : chunks_) cudaFree(c.base);
@@ -115,6 +123,11 @@ PinnedArena::~PinnedArena() {
 void PinnedArena::reset() {
     for (auto &c : chunks_) c.used = 0;
     current_ = 0;
+}
+PinnedArena::Mark PinnedArena::mark() const { return {current_, current_ < chunks_.size() ? chunks_[current_].used : 0}; }
+void PinnedArena::rewind(const Mark &m) {
+    for (size_t i = m.chunk; i < chunks_.size(); ++i) chunks_[i].used = i == m.chunk ? m.used : 0;
+    current_ = m.chunk;
 }
 void *PinnedArena::alloc(size_t bytes) {
     bytes = round_up(bytes ? bytes : 1);
@@ -338,7 +351,8 @@ void *Engine::upload_bytes(const void *src, size_t bytes) {
     const size_t need = (std::max<size_t>(bytes, 1) + 255) / 256 * 256;
     if (up_end_ + need > up_cap_) {
         flush_uploads();
-        up_cap_ = std::max(need, size_t(1) << 20);
+        // (the first chunk is all that most single pairs take)
+        up_cap_ = std::max(need, up_cap_ ? size_t(1) << 20 : size_t(512) << 10);
         up_host_ = static_cast<char *>(pinned_.alloc(up_cap_));
         up_dev_ = static_cast<char *>(arena_.alloc(up_cap_));
         up_begin_ = up_end_ = 0;
@@ -440,6 +454,21 @@ void Engine::begin_batch() {
     arena_.reset();
     pinned_.reset();
     up_cap_ = up_begin_ = up_end_ = 0;
+}
+
+Engine::Phase Engine::begin_phase() {
+    return Phase{arena_.mark(), pinned_.mark(), up_host_, up_dev_, up_cap_, up_end_};
+}
+
+// (what was uploaded before the phase lies before up_end and stays; a chunk
+// that the phase opened goes back with the arenas)
+void Engine::end_phase(const Phase &p) {
+    arena_.rewind(p.arena);
+    pinned_.rewind(p.pinned);
+    up_host_ = p.up_host;
+    up_dev_ = p.up_dev;
+    up_cap_ = p.up_cap;
+    up_begin_ = up_end_ = p.up_end;
 }
 
 void Engine::d2h(void *dst, const void *src, size_t bytes) {
@@ -603,9 +632,11 @@ size_t Engine::pair_footprint(size_t rl, size_t dl, uint32_t sample_rate, bool s
                + 8 * NB * (2 * nfr + 2 * nfd + 4 * width)      // spectrograms, prepared copies, plane
                + np * (8 * 4 * NB * P + 24 * nfd + 8 * (3 * NB + 1) + 16)  // terms, table, DP, stats
                + np * (16 * n_slice + 8 * 4 * NB * (2 * P + 2) + 256);     // realignment slices
-    // The lag searches nominate in f32, 8 bytes a point; the other 8 hold an
-    // exact rerun, or leave room for the exact form's sums and the FMA forms'
-    // spectra (44 KB a frame for up to 2048 frames, once for a batch).
+    // 16 bytes a point: an exact search, or the exact rerun of an f32 search (8
+    // bytes a point, given back before). The FMA forms' spectra (44 KB a 48 kHz
+    // frame of a pass) have what the realignment searches leave, whose
+    // transforms are half of n_slice, and the quarter below; later plans make
+    // their scratch larger only within the footprint (spare in measure_batch).
     b += b / 4 + (size_t(1) << 20);  // job tables, tiles, rounding slack
     return b;
 }
@@ -624,7 +655,7 @@ const void *Engine::upload_tiles(const std::vector<SpecJob> &jobs, int F, int *n
 }
 
 Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc,
-                                           const SpecPlan *before, size_t room) {
+                                           size_t room, const SpecPlan *before, size_t spare) {
     SpecPlan plan;
     plan.rc = &rc;
     for (const SpecJob &j : jobs) plan.frames += (size_t)j.nf;
@@ -645,12 +676,14 @@ Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, con
                 frames[k++] = SpectralFrame{j.sig.base + first, j.out + f, (int32_t)lo, (int32_t)hi, j.nf};
             }
         plan.d_frames = upload(frames);
-        plan.scratch_count = spectral_scratch_count(*rc.spectral, (int)std::max(plan.frames, room));
-        if (before && before->scratch_count >= spectral_scratch_count(*rc.spectral, (int)plan.frames)) {
+        plan.scratch_frames = spectral_scratch_frames(*rc.spectral, (int)std::max(plan.frames, room));
+        const size_t count = spectral_scratch_count(*rc.spectral, plan.scratch_frames);
+        if (before && before->scratch &&
+            (before->scratch_frames >= plan.scratch_frames || count * sizeof(double) > spare)) {
             plan.scratch = before->scratch;
-            plan.scratch_count = before->scratch_count;
+            plan.scratch_frames = before->scratch_frames;
         } else {
-            plan.scratch = arena_.alloc_n<double>(plan.scratch_count);
+            plan.scratch = arena_.alloc_n<double>(count);
         }
         return plan;
     }
@@ -678,7 +711,8 @@ void Engine::run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t
     }
     if (begin) VQB_CUDA(cudaEventRecord(begin, st));
     if (plan.d_frames)
-        launch_spectral(*rc.spectral, rc.spectral_dev, rc.d_fast_coeffs, plan.d_frames, (int)plan.frames, plan.scratch, st);
+        launch_spectral(*rc.spectral, rc.spectral_dev, rc.d_fast_coeffs, plan.d_frames, (int)plan.frames, plan.scratch,
+                        plan.scratch_frames, st);
     else if (opt_.form == kFormExact)
         launch_gammatone(plan.d_jobs, plan.d_tiles, plan.ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, plan.tile, st);
     else
@@ -1054,6 +1088,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
 
     // ---- inputs -----------------------------------------------------------
     std::vector<HostStager::Copy> copies;
+    size_t footprint = 0;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
         s.prep = prepared ? prepared[i] : nullptr;
@@ -1063,6 +1098,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         }
         s.rl = s.prep ? s.prep->len : ref_lens[i];
         s.dl = deg_lens[i];
+        footprint += pair_footprint(s.rl, s.dl, sample_rate, opt_.speech);
         if ((!s.prep && s.rl && !refs[i]) || (s.dl && !degs[i])) {
             s.fail(kInvalid, "signal pointer is NULL");
             continue;
@@ -1148,6 +1184,8 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             if (vad_at[i] != SIZE_MAX) vads[v++].loud = reinterpret_cast<uint8_t *>(d_phase1 + loud_at) + vad_at[i];
     }
     launch_zero(d_phase1, loud_at, stream_);
+    char *h_phase1 = static_cast<char *>(pinned_.alloc(phase1_bytes));
+    Phase phase1;
     std::vector<LagJob> lag_jobs;
     std::vector<size_t> lag_pair;  // pair of each lag job
     // aligned energies (read the lags on the device) of the listed pairs
@@ -1197,7 +1235,9 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         std::vector<size_t> all(n);
         for (size_t i = 0; i < n; ++i) all[i] = i;
         // every upload of the phase goes up with the first flush
-        ref_spec = plan_spectrograms(ref_jobs, rc, nullptr, deg_frames);
+        ref_spec = plan_spectrograms(ref_jobs, rc, deg_frames);
+        // (the reference spectrograms may still run when the phase ends)
+        phase1 = begin_phase();
         const Launches do_sums = plan_sums(sums), do_lags = plan_lag_jobs(lag_jobs, false, d_lstat),
                        do_aligned = plan_aligned(all), do_vad = plan_vad(vads);
         run_gammatone(ref_spec, side_);
@@ -1209,7 +1249,6 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         run(do_aligned);
         run(do_vad);
     }
-    char *h_phase1 = static_cast<char *>(pinned_.alloc(phase1_bytes));
     const int64_t *h_lags = reinterpret_cast<int64_t *>(h_phase1 + lags_at);
     double *h_stats = reinterpret_cast<double *>(h_phase1);
     const int32_t *h_lstat = d_lstat ? reinterpret_cast<int32_t *>(h_phase1 + status_at) : nullptr;
@@ -1217,6 +1256,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     d2h(h_phase1, d_phase1, phase1_bytes);
     record(events_[1]);
     sync();
+    end_phase(phase1);
     {
         // searches the f32 pass left undecided: the exact search, then those
         // pairs' aligned energies again
@@ -1227,6 +1267,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             run(plan_aligned(pairs));
             d2h(h_phase1, d_phase1, phase1_bytes);
             sync();
+            end_phase(phase1);
         }
     }
     for (size_t i = 0; i < n; ++i)
@@ -1247,6 +1288,14 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     std::vector<StatsJob> stat_jobs;
     int max_width = 0, max_offsets = 0;
     size_t npatches = 0;
+    // What the batch may still take of its pairs' footprints, leaving `later`
+    // to later phases and a megabyte a pair to job arrays and rounding.
+    auto spare = [&](size_t later) {
+        const size_t used = arena_.in_use() + later + (n << 20);
+        return footprint > used ? footprint - used : 0;
+    };
+    // a realigned patch: its lag search (P hops, an end's rounding), exact, and its spectrograms
+    const size_t slice_search = 16 * host::fft_size_for(P * H + 2) + 8 * 4 * NB * (2 * P + 2) + 512;
     for (size_t i = 0; i < n; ++i) {
         PairState &s = ps[i];
         if (!s.live) continue;
@@ -1351,7 +1400,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
 
     // ---- 3: spectrograms, prep, NSIM table, DP, match statistics ----------
     // every upload of the phase goes up with the first flush
-    const SpecPlan deg_spec = plan_spectrograms(spec_jobs, rc, &ref_spec);
+    const SpecPlan deg_spec = plan_spectrograms(spec_jobs, rc, 0, &ref_spec, spare(npatches * slice_search));
     const Launches do_prep = plan_prep_jobs(prep_jobs);
     const void *d_scale = upload_bytes(scale_args.data(), scale_args.size());
     const PlaneJob *d_planes = upload(plane_jobs);
@@ -1462,18 +1511,21 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
             }
         }
         // ---- 5: slice lags --------------------------------------------------
+        int64_t *h_sl = static_cast<int64_t *>(pinned_.alloc(slice_bytes));
+        const int32_t *h_sstat = d_sstat ? reinterpret_cast<int32_t *>(h_sl + n_slices) : nullptr;
+        const Phase phase = begin_phase();
         {
             const Launches do_sums = plan_sums(slice_sums), do_lags = plan_lag_jobs(slice_lags, false, d_sstat);
             run(do_sums);
             run(do_lags);
         }
-        int64_t *h_sl = static_cast<int64_t *>(pinned_.alloc(slice_bytes));
-        const int32_t *h_sstat = d_sstat ? reinterpret_cast<int32_t *>(h_sl + n_slices) : nullptr;
         d2h(h_sl, d_slice_lags, slice_bytes);
         sync();
+        end_phase(phase);
         if (!rerun_undecided(slice_lags, h_sstat, false).empty()) {
             d2h(h_sl, d_slice_lags, slice_bytes);
             sync();
+            end_phase(phase);
         }
 
         // ---- 6: trimmed geometry, frame reuse (host) -------------------------
@@ -1527,7 +1579,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
         }
         // ---- 7: realigned spectrograms and statistics ------------------------
         const CopyJob *d_copies = upload(copies);
-        const SpecPlan slice_spec = plan_spectrograms(rjobs, rc, &deg_spec);
+        const SpecPlan slice_spec = plan_spectrograms(rjobs, rc, 0, &deg_spec, spare(0));
         const Launches do_rprep = plan_prep_jobs(rprep);
         const StatsJob *d_rstats = upload(rstats);
         flush_uploads();
@@ -1612,6 +1664,7 @@ void Engine::measure_batch(size_t n, const double *const *refs, const size_t *re
     timing_.prep_ms = elapsed(events_[3], events_[4]);
     timing_.nsim_ms = elapsed(events_[4], events_[5]);
     timing_.realign_ms = n_slices ? elapsed(events_[5], events_[6]) : 0.0;
+    timing_.arena_bytes = arena_.peak();
 }
 
 void Engine::measure_batch_streamed(size_t n, const double *const *refs, const size_t *ref_lens,
@@ -1744,6 +1797,7 @@ void Engine::measure_batch_streamed(size_t n, const double *const *refs, const s
         sum.lag_kernel_ms += t.lag_kernel_ms;
         sum.lag_bytes += t.lag_bytes;
         sum.lag_reruns += t.lag_reruns;
+        sum.arena_bytes = std::max(sum.arena_bytes, t.arena_bytes);
     }
     sum.h2d_bytes += h2d;
     timing_ = sum;

@@ -66,6 +66,7 @@ struct Timing {
     uint64_t lag_reruns = 0;  // f32 lag searches left undecided and rerun exactly
     double lag_kernel_ms = 0;  // the global lag search's kernels (events around them)
     uint64_t lag_bytes = 0;    // their algorithmic DRAM bytes
+    uint64_t arena_bytes = 0;  // the most that the batch held of its arena
 };
 
 // Device memory that grows by whole chunks and is recycled per batch.
@@ -81,6 +82,16 @@ public:
         return static_cast<T *>(alloc(n * sizeof(T)));
     }
     size_t reserved() const;
+    // Bytes in use, and the most at a time since reset().
+    size_t in_use() const { return in_use_; }
+    size_t peak() const { return peak_; }
+    // rewind(mark()) gives back what was taken since the mark (the device must
+    // be done with it).
+    struct Mark {
+        size_t chunk = 0, used = 0, in_use = 0;
+    };
+    Mark mark() const;
+    void rewind(const Mark &m);
 
 private:
     struct Chunk {
@@ -89,6 +100,7 @@ private:
     };
     std::vector<Chunk> chunks_;
     size_t current_ = 0;
+    size_t in_use_ = 0, peak_ = 0;
 };
 
 // Page-locked host memory with the same policy.
@@ -101,6 +113,11 @@ public:
     T *alloc_n(size_t n) {
         return static_cast<T *>(alloc(n * sizeof(T)));
     }
+    struct Mark {
+        size_t chunk = 0, used = 0;
+    };
+    Mark mark() const;
+    void rewind(const Mark &m);
 
 private:
     struct Chunk {
@@ -261,15 +278,17 @@ private:
         uint64_t rms = 0;
         const SpectralFrame *d_frames = nullptr;  // the spectral kernels' frames, or
         double *scratch = nullptr;
-        size_t scratch_count = 0;
+        int scratch_frames = 0;
         const SpecJob *d_jobs = nullptr;  // the recurrence kernels' jobs and tiles of `tile` frames
         const void *d_tiles = nullptr;
         int ntiles = 0, tile = 0;
     };
-    // before: a plan whose launches come before this one's, whose scratch is
-    // used again if it is large enough; room: frames to make the scratch large enough for
-    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, const SpecPlan *before = nullptr,
-                               size_t room = 0);
+    // room: frames to make the scratch large enough for. before: a plan whose
+    // launches come before this one's, whose scratch is used again: in several
+    // passes where it holds fewer frames and a new one would take more than
+    // `spare` bytes.
+    SpecPlan plan_spectrograms(const std::vector<SpecJob> &jobs, const RateCache &rc, size_t room = 0,
+                               const SpecPlan *before = nullptr, size_t spare = 0);
     void run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t begin = nullptr,
                           cudaEvent_t end = nullptr);
     const void *upload_tiles(const std::vector<SpecJob> &jobs, int F, int *ntiles);
@@ -295,6 +314,17 @@ private:
     void *upload_bytes(const void *src, size_t bytes);
     void flush_uploads();
     void begin_batch();
+    // What a phase takes for itself (device scratch, job arrays) from
+    // begin_phase on, end_phase gives back once the main stream has been
+    // waited for: the phases after it take the same memory.
+    struct Phase {
+        Arena::Mark arena;
+        PinnedArena::Mark pinned;
+        char *up_host, *up_dev;
+        size_t up_cap, up_end;
+    };
+    Phase begin_phase();
+    void end_phase(const Phase &p);
     void d2h(void *dst, const void *src, size_t bytes);
     void sync();
     void record(cudaEvent_t e);

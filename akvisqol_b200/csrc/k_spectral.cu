@@ -477,12 +477,14 @@ constexpr int kWide = 1024;   // frames from which a tail task takes four bands
 
 // Frames of a launch: as many as leave their spectra in the L2 (67 MB).
 int chunk_frames(const SpectralTables &t) { return 2048 << (12 - t.log_m); }
-int chunk_cap(const SpectralTables &t, int nframes) { return (std::min(nframes, chunk_frames(t)) + 63) / 64 * 64; }
 
 }  // namespace
 
-size_t spectral_scratch_count(const SpectralTables &t, int nframes) {
-    return (size_t)chunk_cap(t, nframes) * (size_t)(t.row + 32 * t.slots + t.nbp * t.splits);
+int spectral_scratch_frames(const SpectralTables &t, int nframes) {
+    return (std::min(nframes, chunk_frames(t)) + 31) / 32 * 32;  // whole tiles
+}
+size_t spectral_scratch_count(const SpectralTables &t, int scratch_frames) {
+    return (size_t)scratch_frames * (size_t)(t.row + 32 * t.slots + t.nbp * t.splits);
 }
 
 int spectral_frame_count(int nframes) { return (nframes + 63) / 64 * 64; }
@@ -492,15 +494,14 @@ void spectral_init_attributes() {
 }
 
 void launch_spectral(const SpectralTables &t, const SpectralDevice &d, const FastBandCoeffs *d_coeffs,
-                     const SpectralFrame *d_frames, int nframes, double *d_scratch, cudaStream_t s) {
-    const int cap = chunk_cap(t, nframes);
+                     const SpectralFrame *d_frames, int nframes, double *d_scratch, int scratch_frames, cudaStream_t s) {
+    const int cap = scratch_frames;
     double *power = d_scratch, *tail_part = power + (size_t)cap * t.row,
            *power_part = tail_part + (size_t)cap * 32 * t.slots;
     const int M = 1 << t.log_m;
     const size_t smem = (size_t)(M + M / 16) * sizeof(double2);
-    const int chunk = chunk_frames(t);
-    for (int f0 = 0; f0 < nframes; f0 += chunk) {
-        const int n = std::min(chunk, nframes - f0);
+    for (int f0 = 0; f0 < nframes; f0 += cap) {
+        const int n = std::min(cap, nframes - f0);
         const SpectralFrame *fr = d_frames + f0;
         if (t.log_m == 12)
             spectrum_kernel<12><<<n, M / 16, smem, s>>>(fr, d.hann, d.twiddles, power, t.row, t.window);

@@ -176,11 +176,14 @@ struct SpectralDevice {  // SpectralTables on the device
 };
 void spectral_init_attributes();
 // d_frames: spectral_frame_count(nframes) entries, empty ones (lo = hi = 0)
-// behind the last; d_scratch: spectral_scratch_count doubles.
+// behind the last; d_scratch: spectral_scratch_count doubles for
+// scratch_frames frames, those of a pass. spectral_scratch_frames: a pass's
+// frames for nframes.
 int spectral_frame_count(int nframes);
-size_t spectral_scratch_count(const SpectralTables &t, int nframes);
+int spectral_scratch_frames(const SpectralTables &t, int nframes);
+size_t spectral_scratch_count(const SpectralTables &t, int scratch_frames);
 void launch_spectral(const SpectralTables &t, const SpectralDevice &d, const FastBandCoeffs *d_coeffs,
-                     const SpectralFrame *d_frames, int nframes, double *d_scratch, cudaStream_t s);
+                     const SpectralFrame *d_frames, int nframes, double *d_scratch, int scratch_frames, cudaStream_t s);
 
 // k_gammatone_fast.cu: the FMA forms' recurrence (tiles as fill_gammatone_tile
 // writes them, of gammatone_staged_frames_per_cta() frames).

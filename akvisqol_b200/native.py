@@ -142,6 +142,7 @@ def _load() -> ctypes.CDLL:
                                                    POINTER(c_void_p)]),
         "visqol_b200_trace_free": (None, [POINTER(Trace)]),
         "visqol_b200_last_timing": (c_int, [c_void_p, POINTER(Timing)]),
+        "visqol_b200_last_batch_bytes": (c_int, [c_void_p, POINTER(c_uint64)]),
         "visqol_b200_device_info": (c_int, [c_int, c_char_p, c_size_t, POINTER(c_int), POINTER(c_int),
                                             POINTER(c_int)]),
         "visqol_b200_spectrogram": (c_int, [c_size_t, D, D, c_size_t, c_size_t, D, c_size_t, D, SZ]),
@@ -199,7 +200,8 @@ EXPORTS = [
     "visqol_abi_version", "visqol_version", "visqol_last_error", "visqol_available_backends",
     "visqol_options_default", "visqol_create", "visqol_destroy", "visqol_measure", "visqol_measure_files",
     "visqol_measure_batch", "visqol_measure_files_batch", "visqol_result_free",
-    "visqol_b200_measure_batch", "visqol_b200_measure_batch_grad", "visqol_b200_trace_free", "visqol_b200_last_timing", "visqol_b200_device_info",
+    "visqol_b200_measure_batch", "visqol_b200_measure_batch_grad", "visqol_b200_trace_free", "visqol_b200_last_timing", "visqol_b200_last_batch_bytes",
+    "visqol_b200_device_info",
     "visqol_b200_spectrogram", "visqol_b200_envelope_lag", "visqol_b200_best_lag", "visqol_b200_fft",
     "visqol_b200_signal_sums",
     "visqol_b200_lag_search", "visqol_b200_refine_lag", "visqol_b200_nsim_quotient",
@@ -464,6 +466,12 @@ class Context:
         t = Timing()
         _check(lib.visqol_b200_last_timing(self._handle, ctypes.byref(t)))
         return {name: getattr(t, name) for name, _ in Timing._fields_}
+
+    def last_batch_bytes(self) -> int:
+        """The most device memory a lane held in its arena during the last batch."""
+        b = c_uint64()
+        _check(lib.visqol_b200_last_batch_bytes(self._handle, ctypes.byref(b)))
+        return b.value
 
 
 def free(result) -> None:

@@ -93,6 +93,9 @@ int visqol_b200_measure_batch_grad(visqol_ctx *ctx, size_t n,
                                    uint32_t sample_rate, uint32_t flags,
                                    visqol_result **out, int32_t *status, double *const *grads);
 int visqol_b200_last_timing(visqol_ctx *ctx, visqol_b200_timing *out);
+/* The most device memory that one of the context's lanes held in its arena
+ * during the last batch (what visqol_b200_pair_footprint bounds for a pair). */
+int visqol_b200_last_batch_bytes(visqol_ctx *ctx, uint64_t *bytes);
 
 /* ---- prepared references ---------------------------------------------------
  * The reference-side work (samples, envelope statistics and spectrogram on
