@@ -36,6 +36,7 @@
 
 #include "grad_host.h"
 #include "kernels.h"
+#include "shared_tables.h"
 #include "threads.h"
 
 namespace vqb {
@@ -300,11 +301,11 @@ struct Engine::TwiddleTable {
 const Engine::Twiddles &Engine::twiddles(size_t n) {
     auto it = twiddles_.find(n);
     if (it != twiddles_.end()) return it->second->view;
-    static std::mutex mu;
-    static std::map<std::pair<int, size_t>, std::weak_ptr<const TwiddleTable>> shared;
-    std::lock_guard<std::mutex> lock(mu);
-    std::weak_ptr<const TwiddleTable> &entry = shared[{device_, n}];
-    if (auto held = entry.lock()) return (twiddles_[n] = std::move(held))->view;
+    static SharedTables<std::pair<int, size_t>, TwiddleTable> shared;
+    return (twiddles_[n] = shared.get({device_, n}, [&] { return make_twiddles(n); }))->view;
+}
+
+std::shared_ptr<const Engine::TwiddleTable> Engine::make_twiddles(size_t n) {
     // top[k] = W_n^k (k < n/2), then the block passes' W_B^k = top[k * n/B].
     // then the fused lag search's stage-major column twiddles.
     std::vector<double2> t = host::twiddles(n);
@@ -334,9 +335,7 @@ const Engine::Twiddles &Engine::twiddles(size_t n) {
     }
     // (on the device before another engine's streams see it)
     const Twiddles tw{d, d + half, d + cols_at, d + stages_at, d32, d32 + (cols_at - half), d32 + (stages_at - half)};
-    auto made = std::make_shared<const TwiddleTable>(device_, d, tw);
-    entry = made;
-    return (twiddles_[n] = std::move(made))->view;
+    return std::make_shared<const TwiddleTable>(device_, d, tw);
 }
 
 template <class T>

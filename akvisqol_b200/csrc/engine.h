@@ -238,6 +238,7 @@ public:
     };
     struct TwiddleTable;
     const Twiddles &twiddles(size_t n);
+    std::shared_ptr<const TwiddleTable> make_twiddles(size_t n);
 
 private:
     struct RateCache {

@@ -7,10 +7,11 @@
 #include <array>
 #include <atomic>
 #include <cmath>
-#include <map>
+#include <deque>
 #include <mutex>
 #include <thread>
 
+#include "shared_tables.h"
 #include "threads.h"
 
 namespace vqb {
@@ -288,19 +289,21 @@ std::shared_ptr<const SpectralTables> build(const std::vector<BandCoeffs> &run, 
 bool spectral_window(size_t window) { return window > 512 && window <= 4096; }
 
 std::shared_ptr<const SpectralTables> spectral_tables(const std::vector<BandCoeffs> &run, size_t window) {
-    // shared by the process's engines; a program uses a few rates
+    // shared by the process's engines, and kept behind the last of them for
+    // the next context (a program uses a few rates; the longest kept goes first)
+    static SharedTables<std::vector<double>, SpectralTables> shared;
     static std::mutex mu;
-    static std::map<std::vector<double>, std::shared_ptr<const SpectralTables>> cache;
+    static std::deque<std::shared_ptr<const SpectralTables>> kept;
     std::vector<double> key{(double)window};
     for (const BandCoeffs &c : run)
         for (double v : {c.s1n0, c.s1n1, c.s2n1, c.s3n1, c.s4n1, c.ca0, c.d1, c.d2}) key.push_back(v);
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it == cache.end()) {
-        if (cache.size() >= 16) cache.clear();
-        it = cache.emplace(key, build(run, window)).first;
-    }
-    return it->second;
+    return shared.get(key, [&] {
+        auto made = build(run, window);
+        std::lock_guard<std::mutex> lock(mu);
+        kept.push_back(made);
+        if (kept.size() > 16) kept.pop_front();
+        return made;
+    });
 }
 
 }  // namespace vqb
