@@ -687,10 +687,11 @@ Engine::SpecPlan Engine::plan_spectrograms(const std::vector<SpecJob> &jobs, con
         return plan;
     }
     if (opt_.form == kFormExact) {
-        // a rule's shape (VISQOL_TUNE_0 may fix another)
-        const std::vector<int> shapes = gammatone_frames_shapes(nbi);
-        plan.tile = tuned(kTuneGammatone, opt_.form, nbi, {gammatone_frames_per_cta(nbi, (int64_t)plan.frames)},
-                          [](int) {}, stream_, &shapes);
+        plan.tile = gammatone_frames_per_cta(nbi, (int64_t)plan.frames);
+        if (const char *env = std::getenv("VISQOL_TUNE_0")) {  // fixes one of the shapes with a thread a band
+            const std::vector<int> shapes = gammatone_frames_shapes(nbi);
+            if (std::find(shapes.begin(), shapes.end(), std::atoi(env)) != shapes.end()) plan.tile = std::atoi(env);
+        }
     } else {
         plan.tile = gammatone_staged_frames_per_cta();
     }
@@ -737,13 +738,12 @@ bool autotune_enabled() {
 }  // namespace
 
 int Engine::tuned(int kernel, int a, int b, const std::vector<int> &candidates,
-                  const std::function<void(int)> &launch, cudaStream_t st, const std::vector<int> *allowed) {
+                  const std::function<void(int)> &launch, cudaStream_t st) {
     // VISQOL_TUNE_<kernel>=<choice> fixes a kernel class's shape (one of its
     // candidates), e.g. to check that every shape gives the same results.
     if (const char *env = std::getenv(("VISQOL_TUNE_" + std::to_string(kernel)).c_str())) {
         const int forced = std::atoi(env);
-        const std::vector<int> &ok = allowed ? *allowed : candidates;
-        if (std::find(ok.begin(), ok.end(), forced) != ok.end()) return forced;
+        if (std::find(candidates.begin(), candidates.end(), forced) != candidates.end()) return forced;
     }
     if (!autotune_enabled() || candidates.size() < 2) return candidates.at(0);
     const auto key = std::make_tuple(device_, kernel, a, b);
@@ -1922,12 +1922,11 @@ void Engine::gradients(detail::PairState *ps, size_t n, const size_t *deg_lens, 
                                    (int64_t)rp.nf, upload(sg.g), d_g[sg.pair] + rp.dl.base});
     }
     if (!jobs.empty()) {
-        const int F = gammatone_bwd_frames_per_cta();
         const size_t tsz = gammatone_tile_size();
         std::vector<char> tiles;
         int ntiles = 0;
         for (size_t j = 0; j < jobs.size(); ++j)
-            for (int64_t f = 0; f < jobs[j].nf; f += F, ++ntiles) {
+            for (int64_t f = 0; f < jobs[j].nf; ++f, ++ntiles) {
                 tiles.resize(tiles.size() + tsz);
                 fill_gammatone_tile(tiles.data() + tiles.size() - tsz, (int)j, (int)f);
             }

@@ -265,13 +265,11 @@ private:
     // caller's jobs at first use per device (launch(c) launches them with
     // shape c on st), then reused; candidates[0] when autotuning is off.
     enum TuneKernel {
-        kTuneGammatone = 0,
         kTuneLagColumns = 2
     };
-    // VISQOL_TUNE_<kernel> may fix the shape to one of `allowed` (default:
-    // the candidates).
+    // VISQOL_TUNE_<kernel> may fix the shape to one of the candidates.
     int tuned(int kernel, int a, int b, const std::vector<int> &candidates, const std::function<void(int)> &launch,
-              cudaStream_t st, const std::vector<int> *allowed = nullptr);
+              cudaStream_t st);
     // Gammatone spectrograms of the jobs in this engine's form, on stream st.
     struct SpecPlan {
         const RateCache *rc = nullptr;

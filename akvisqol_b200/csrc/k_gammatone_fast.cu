@@ -1,8 +1,8 @@
 // Gammatone filterbank spectrograms of the FMA forms by the recurrence itself:
 // the cascade of four biquads per (frame, band) of the exact kernel (reference
 // src/gammatone.zig:268-306) without its operation order. It serves the
-// windows and band counts that the spectral kernels (k_spectral.cu) do not:
-// sample rates above 51.2 kHz or up to 6.4 kHz.
+// windows that the spectral kernels (k_spectral.cu) do not: sample rates above
+// 51.2 kHz or up to 6.4 kHz.
 //
 // Each biquad runs in direct form I with its numerator normalised to
 // 1 + beta z^-1 (the four numerator gains and the band gain become one
@@ -194,12 +194,8 @@ void launch_gammatone_staged(const SpecJob *d_jobs, const void *d_tiles, int nti
     const Tile *t = static_cast<const Tile *>(d_tiles);
     if (nb > 24)
         gammatone_staged_kernel<256><<<ntiles, 256, 0, s>>>(d_jobs, t, d_coeffs, nb, d_hann, window, hop);
-    else if (nb > 16)
-        gammatone_staged_kernel<192><<<ntiles, 192, 0, s>>>(d_jobs, t, d_coeffs, nb, d_hann, window, hop);
-    else if (nb > 8)
-        gammatone_staged_kernel<128><<<ntiles, 128, 0, s>>>(d_jobs, t, d_coeffs, nb, d_hann, window, hop);
     else
-        gammatone_staged_kernel<64><<<ntiles, 64, 0, s>>>(d_jobs, t, d_coeffs, nb, d_hann, window, hop);
+        gammatone_staged_kernel<192><<<ntiles, 192, 0, s>>>(d_jobs, t, d_coeffs, nb, d_hann, window, hop);
     launch_counter() += 1;
 }
 

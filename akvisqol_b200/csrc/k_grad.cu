@@ -229,8 +229,6 @@ __global__ void __launch_bounds__(kMaxWarps * 32) gammatone_bwd_kernel(const Gra
 
 }  // namespace
 
-int gammatone_bwd_frames_per_cta() { return 1; }
-
 size_t gammatone_bwd_scratch_count(int ntiles, int window) {
     return (size_t)ntiles * kMaxWarps * 32 * (size_t)((window + kBlock - 1) / kBlock) * kState;
 }

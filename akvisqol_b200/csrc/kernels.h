@@ -185,17 +185,16 @@ size_t spectral_scratch_count(const SpectralTables &t, int scratch_frames);
 void launch_spectral(const SpectralTables &t, const SpectralDevice &d, const FastBandCoeffs *d_coeffs,
                      const SpectralFrame *d_frames, int nframes, double *d_scratch, int scratch_frames, cudaStream_t s);
 
-// k_gammatone_fast.cu: the FMA forms' recurrence (tiles as fill_gammatone_tile
-// writes them, of gammatone_staged_frames_per_cta() frames).
+// k_gammatone_fast.cu: the FMA forms' recurrence, 17 to 32 bands (tiles as
+// fill_gammatone_tile writes them, of gammatone_staged_frames_per_cta() frames).
 int gammatone_staged_frames_per_cta();
 void fill_fast_band_coeffs(const BandCoeffs *run, int nb, FastBandCoeffs *out);
 void launch_gammatone_staged(const SpecJob *d_jobs, const void *d_tiles, int ntiles, const FastBandCoeffs *d_coeffs,
                              int nb, const double *d_hann, int window, int hop, cudaStream_t s);
 
 // k_grad.cu: the gammatone spectrogram's reverse (FP64-FMA arithmetic).
-// Tiles as fill_gammatone_tile writes them, of gammatone_bwd_frames_per_cta()
-// frames; d_scratch holds gammatone_bwd_scratch_count(ntiles, window) doubles.
-int gammatone_bwd_frames_per_cta();
+// Tiles as fill_gammatone_tile writes them, of one frame each; d_scratch holds
+// gammatone_bwd_scratch_count(ntiles, window) doubles.
 size_t gammatone_bwd_scratch_count(int ntiles, int window);
 void launch_gammatone_bwd(const GradSpecJob *d_jobs, const void *d_tiles, int ntiles, const FastBandCoeffs *d_coeffs,
                           int nb, const double *d_hann, int window, int hop, double *d_scratch, cudaStream_t s);
