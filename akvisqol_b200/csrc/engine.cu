@@ -205,7 +205,6 @@ Engine::~Engine() {
         cudaFree(kv.second.d_coeffs);
         cudaFree(kv.second.d_fast_coeffs);
         cudaFree(kv.second.d_hann);
-        cudaFree(kv.second.d_spectral);
     }
     for (auto e : events_) cudaEventDestroy(e);
     for (auto e : gt_events_)
@@ -227,6 +226,36 @@ void Engine::release_device_memory() {
         slot_bytes_[k] = 0;
     }
 }
+
+// Device memory of a table that engines share.
+struct TableMemory {
+    int device;
+    void *base = nullptr;
+    TableMemory(int dev, size_t bytes) : device(dev) { VQB_CUDA(cudaMalloc(&base, bytes)); }
+    TableMemory(const TableMemory &) = delete;
+    TableMemory &operator=(const TableMemory &) = delete;
+    ~TableMemory() {
+        int cur = 0;
+        cudaGetDevice(&cur);
+        cudaSetDevice(device);
+        cudaFree(base);
+        cudaSetDevice(cur);
+    }
+};
+
+// Tables on a device, for as long as an engine there holds them, once for all
+// lanes: a transform size's twiddles (2^20 points: ~25 ms of sines and 24 MB),
+// a rate's spectral tables (~4.5 MB at 48 kHz).
+struct Engine::TwiddleTable {
+    TableMemory memory;
+    Twiddles view{};
+    TwiddleTable(int device, size_t bytes) : memory(device, bytes) {}
+};
+struct Engine::SpectralOnDevice {
+    TableMemory memory;
+    SpectralDevice view;
+    SpectralOnDevice(int device, size_t bytes) : memory(device, bytes) {}
+};
 
 const Engine::RateCache &Engine::rate_cache(uint32_t sr) {
     auto it = rates_.find(sr);
@@ -250,53 +279,41 @@ const Engine::RateCache &Engine::rate_cache(uint32_t sr) {
         VQB_CUDA(cudaMemcpyAsync(rc.d_hann, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, stream_));
     if (opt_.form != kFormExact && spectral_window(rc.geo.window)) {
         rc.spectral = spectral_tables(rc.fb.run, rc.geo.window);
-        const SpectralTables &t = *rc.spectral;
-        // one allocation, each table at a 256-byte boundary
-        size_t bytes = 0;
-        std::vector<std::pair<const void *, size_t>> parts;
-        std::vector<size_t> at;
-        auto add = [&](const auto &v) {
-            parts.emplace_back(v.data(), v.size() * sizeof(v[0]));
-            at.push_back(bytes);
-            bytes += (parts.back().second + 255) / 256 * 256;
-        };
-        add(t.hann), add(t.weights), add(t.tails), add(t.twiddles), add(t.wide), add(t.narrow), add(t.quad_slot),
-            add(t.quad_segs);
-        VQB_CUDA(cudaMalloc(&rc.d_spectral, bytes));
-        char *d = static_cast<char *>(rc.d_spectral);
-        for (size_t i = 0; i < parts.size(); ++i)
-            VQB_CUDA(cudaMemcpyAsync(d + at[i], parts[i].first, parts[i].second, cudaMemcpyHostToDevice, stream_));
-        rc.spectral_dev.hann = reinterpret_cast<const double *>(d + at[0]);
-        rc.spectral_dev.weights = reinterpret_cast<const double *>(d + at[1]);
-        rc.spectral_dev.tails = reinterpret_cast<const double *>(d + at[2]);
-        rc.spectral_dev.twiddles = reinterpret_cast<const double2 *>(d + at[3]);
-        rc.spectral_dev.wide = reinterpret_cast<const SpectralTask *>(d + at[4]);
-        rc.spectral_dev.narrow = reinterpret_cast<const SpectralTask *>(d + at[5]);
-        rc.spectral_dev.quad_slot = reinterpret_cast<const int32_t *>(d + at[6]);
-        rc.spectral_dev.quad_segs = reinterpret_cast<const int32_t *>(d + at[7]);
+        static SharedTables<std::pair<int, std::vector<double>>, SpectralOnDevice> shared;
+        rc.spectral_dev = shared.get({device_, rc.spectral->key}, [&] { return upload_spectral(*rc.spectral); });
     }
     VQB_CUDA(cudaStreamSynchronize(stream_));
     return rates_.emplace(sr, std::move(rc)).first->second;
 }
 
-// A size's tables on a device, for as long as an engine there holds them:
-// formed once for all lanes (2^20 points: ~25 ms of sines and 24 MB, which
-// every lane of every mode would pay and keep for itself).
-struct Engine::TwiddleTable {
-    int device;
-    double2 *base;
-    Twiddles view;
-    TwiddleTable(int dev, double2 *d, const Twiddles &v) : device(dev), base(d), view(v) {}
-    TwiddleTable(const TwiddleTable &) = delete;
-    TwiddleTable &operator=(const TwiddleTable &) = delete;
-    ~TwiddleTable() {
-        int cur = 0;
-        cudaGetDevice(&cur);
-        cudaSetDevice(device);
-        cudaFree(base);
-        cudaSetDevice(cur);
-    }
-};
+std::shared_ptr<const Engine::SpectralOnDevice> Engine::upload_spectral(const SpectralTables &t) {
+    // one allocation, each table at a 256-byte boundary
+    size_t bytes = 0;
+    std::vector<std::pair<const void *, size_t>> parts;
+    std::vector<size_t> at;
+    auto add = [&](const auto &v) {
+        parts.emplace_back(v.data(), v.size() * sizeof(v[0]));
+        at.push_back(bytes);
+        bytes += (parts.back().second + 255) / 256 * 256;
+    };
+    add(t.hann), add(t.weights), add(t.tails), add(t.twiddles), add(t.wide), add(t.narrow), add(t.quad_slot),
+        add(t.quad_segs);
+    auto made = std::make_shared<SpectralOnDevice>(device_, bytes);
+    const char *d = static_cast<char *>(made->memory.base);
+    for (size_t i = 0; i < parts.size(); ++i)
+        VQB_CUDA(cudaMemcpyAsync(static_cast<char *>(made->memory.base) + at[i], parts[i].first, parts[i].second,
+                                 cudaMemcpyHostToDevice, stream_));
+    made->view.hann = reinterpret_cast<const double *>(d + at[0]);
+    made->view.weights = reinterpret_cast<const double *>(d + at[1]);
+    made->view.tails = reinterpret_cast<const double *>(d + at[2]);
+    made->view.twiddles = reinterpret_cast<const double2 *>(d + at[3]);
+    made->view.wide = reinterpret_cast<const SpectralTask *>(d + at[4]);
+    made->view.narrow = reinterpret_cast<const SpectralTask *>(d + at[5]);
+    made->view.quad_slot = reinterpret_cast<const int32_t *>(d + at[6]);
+    made->view.quad_segs = reinterpret_cast<const int32_t *>(d + at[7]);
+    VQB_CUDA(cudaStreamSynchronize(stream_));  // (on the device before another engine's streams see it)
+    return made;
+}
 
 const Engine::Twiddles &Engine::twiddles(size_t n) {
     auto it = twiddles_.find(n);
@@ -325,8 +342,8 @@ std::shared_ptr<const Engine::TwiddleTable> Engine::make_twiddles(size_t n) {
     for (size_t k = half; k < t.size(); ++k) t32[k - half] = make_float2((float)t[k].x, (float)t[k].y);
     // one allocation: the f64 tables, then the f32 ones at a 16-byte boundary
     const size_t bytes64 = std::max<size_t>(1, t.size()) * sizeof(double2);
-    double2 *d = nullptr;
-    VQB_CUDA(cudaMalloc(&d, bytes64 + std::max<size_t>(1, t32.size()) * sizeof(float2)));
+    auto made = std::make_shared<TwiddleTable>(device_, bytes64 + std::max<size_t>(1, t32.size()) * sizeof(float2));
+    double2 *d = static_cast<double2 *>(made->memory.base);
     float2 *d32 = reinterpret_cast<float2 *>(reinterpret_cast<char *>(d) + bytes64);
     if (!t.empty()) {
         VQB_CUDA(cudaMemcpyAsync(d, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, stream_));
@@ -334,8 +351,8 @@ std::shared_ptr<const Engine::TwiddleTable> Engine::make_twiddles(size_t n) {
         VQB_CUDA(cudaStreamSynchronize(stream_));
     }
     // (on the device before another engine's streams see it)
-    const Twiddles tw{d, d + half, d + cols_at, d + stages_at, d32, d32 + (cols_at - half), d32 + (stages_at - half)};
-    return std::make_shared<const TwiddleTable>(device_, d, tw);
+    made->view = Twiddles{d, d + half, d + cols_at, d + stages_at, d32, d32 + (cols_at - half), d32 + (stages_at - half)};
+    return made;
 }
 
 template <class T>
@@ -711,7 +728,7 @@ void Engine::run_spectrograms(const SpecPlan &plan, cudaStream_t st, cudaEvent_t
     }
     if (begin) VQB_CUDA(cudaEventRecord(begin, st));
     if (plan.d_frames)
-        launch_spectral(*rc.spectral, rc.spectral_dev, rc.d_fast_coeffs, plan.d_frames, (int)plan.frames, plan.scratch,
+        launch_spectral(*rc.spectral, rc.spectral_dev->view, rc.d_fast_coeffs, plan.d_frames, (int)plan.frames, plan.scratch,
                         plan.scratch_frames, st);
     else if (opt_.form == kFormExact)
         launch_gammatone(plan.d_jobs, plan.d_tiles, plan.ntiles, rc.d_coeffs, nbi, rc.d_hann, W, H, plan.tile, st);

@@ -239,6 +239,8 @@ public:
     struct TwiddleTable;
     const Twiddles &twiddles(size_t n);
     std::shared_ptr<const TwiddleTable> make_twiddles(size_t n);
+    struct SpectralOnDevice;
+    std::shared_ptr<const SpectralOnDevice> upload_spectral(const SpectralTables &t);
 
 private:
     struct RateCache {
@@ -249,8 +251,7 @@ private:
         double *d_hann = nullptr;
         // FMA forms, windows the spectral kernels serve
         std::shared_ptr<const SpectralTables> spectral;
-        SpectralDevice spectral_dev;
-        void *d_spectral = nullptr;
+        std::shared_ptr<const SpectralOnDevice> spectral_dev;
     };
     // A phase's work is planned first (device buffers, job arrays through
     // upload) and launched after, so that its uploads go up in one copy: run

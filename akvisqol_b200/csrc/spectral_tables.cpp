@@ -190,7 +190,7 @@ int bitrev(int v, int bits) {
     return r;
 }
 
-std::shared_ptr<const SpectralTables> build(const std::vector<BandCoeffs> &run, size_t window) {
+std::shared_ptr<SpectralTables> build(const std::vector<BandCoeffs> &run, size_t window) {
     auto t = std::make_shared<SpectralTables>();
     int log_m = 10;
     while (((size_t)1 << log_m) < window) ++log_m;
@@ -299,6 +299,7 @@ std::shared_ptr<const SpectralTables> spectral_tables(const std::vector<BandCoef
         for (double v : {c.s1n0, c.s1n1, c.s2n1, c.s3n1, c.s4n1, c.ca0, c.d1, c.d2}) key.push_back(v);
     return shared.get(key, [&] {
         auto made = build(run, window);
+        made->key = key;
         std::lock_guard<std::mutex> lock(mu);
         kept.push_back(made);
         if (kept.size() > 16) kept.pop_front();

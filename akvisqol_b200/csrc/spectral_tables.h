@@ -23,6 +23,7 @@ struct SpectralTask {
 
 // Everything that depends on the filterbank and the window alone.
 struct SpectralTables {
+    std::vector<double> key;  // what they depend on: the window and the bands' coefficients
     int log_m = 0;        // complex transform size M = 2^log_m, M >= window
     int nb = 0, nbp = 0;  // bands, padded to a multiple of 8
     int window = 0;
