@@ -597,8 +597,8 @@ void vqb::set_last_error(const std::string &message) { set_error(message); }
 int vqb::engine_options(const visqol_options &o, Options *opt, std::shared_ptr<const host::Svr> *svr,
                         std::shared_ptr<const host::LatticeMapper> *lattice, std::string *message) {
     // EXACT (and AUTO, which resolves to exact on a device with native f64)
-    // reproduce the CPU path; FAST runs the gammatone's later stages in f32;
-    // BALANCED keeps f64 throughout but with FMA and reassociated sums.
+    // reproduce the CPU path; FAST and BALANCED run in f64 with FMA and
+    // reassociated sums.
     opt->form = o.precision == VISQOL_PRECISION_FAST       ? kFormF32
                 : o.precision == VISQOL_PRECISION_BALANCED ? kFormF64
                                                            : kFormExact;

@@ -404,8 +404,9 @@ bool HostStager::pageable(const void *p) {
 
 // The driver's own copy from pageable memory fills its staging buffers on
 // one thread. Four threads fill page-locked pieces of 512 KB, each with one in
-// flight while it fills the other: a minute's pair (46 MB) 4.1 to 2.1 ms, at
-// the link's 25 GB/s. Below 16 MB the driver's copy is as fast (7.7 MB 0.32
+// flight while it fills the other: a minute's pair (46 MB) 4.1 to 2.1 ms, the
+// 22 GB/s that four copying threads reach (the link carries 56 from
+// page-locked memory). Below 16 MB the driver's copy is as fast (7.7 MB 0.32
 // ms against 0.44).
 void HostStager::run(int device, cudaStream_t stream, const std::vector<Copy> &copies, size_t groups,
                      const std::function<void(size_t)> &issued) {

@@ -220,7 +220,7 @@ public:
     // Single-stage entry points (device buffers, exact form).
     void spectrogram(const host::Filterbank &fb, const double *d_hann, size_t window, size_t hop, const double *d_x,
                      size_t len, double *d_out, size_t nf);
-    // status_out (optional, njobs): FP32 form, 1 where the f32 search left
+    // status_out (optional, njobs): 1 where the f32 search left
     // the job to the exact one.
     void lags(size_t njobs, const VSig *a, const VSig *b, bool raw, int64_t *h_lags, int32_t *status_out = nullptr,
               float *d_corr = nullptr);

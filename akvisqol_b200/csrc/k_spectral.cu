@@ -20,7 +20,11 @@
 // All of it in f64 (the tables are formed in wider arithmetic). Against the recurrence run in extended precision the RMS
 // is off by 1.3e-14 rms and 1.2e-13 at most over music, speech, low-passed
 // and quantised frames and onsets, where the recurrence in f64 FMAs is off by
-// 2.8e-14 and 3.5e-13: sums of positive terms, and no long recurrence.
+// 2.8e-14 and 3.5e-13: no long recurrence, and but for the lowest bands sums of
+// positive terms. (Those bands' weights change sign, the autocorrelation
+// being cut at the window: where a frame is one high tone cut short and the
+// band 45 dB of RMS below it, 21 bands at 16 kHz, the difference is off by
+// 6e-12 at most, the recurrence by 2e-12.)
 //
 // Work per 48 kHz frame (W = 3840, 32 bands) in f64 multiply-adds: the
 // transform ~185 k, the band sums 131 k, the tails 420 k: 0.74 M, where the

@@ -22,7 +22,7 @@ using real = long double;
 constexpr real kPi = 3.141592653589793238462643383279502884L;
 constexpr int kSegment = 480;   // samples of a kind 0 task, at most
 constexpr int kSplit = 512;     // spectrum entries of a kind 1 task
-constexpr real kReach = 40.0L;  // a tail functional reaches back kReach / alpha samples (then below 2^-57 (40^3 / 6))
+constexpr real kReach = 40.0L;  // a tail functional reaches back kReach / alpha samples (its weights then below e^-40 40^3 / 6 = 4.5e-14)
 constexpr size_t kAnchor = 32;  // samples, a power of two
 constexpr real kWrap = 50.0L;   // a band's response has died out after kWrap / alpha samples
 

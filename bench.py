@@ -40,8 +40,8 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRICS = {
-    "fast": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), FP32 form, 1 B200",
-    "balanced": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), FP64 FMA form, 1 B200",
+    "fast": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), FAST form (f64 with FMA), 1 B200",
+    "balanced": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), BALANCED form (f64 with FMA), 1 B200",
     "exact": "ViSQOL pairs/s (audio mode, 10 s 48 kHz pairs), exact FP64 form, 1 B200",
 }
 DTYPES = {"fast": "f64 (FMA); the lag search's nominating transform in f32, its rescoring in f64",

@@ -63,7 +63,7 @@ typedef struct {
     uint64_t host_syncs;
     double lag_kernel_ms;          /* the global lag search's kernels, first to last */
     uint64_t lag_bytes;            /* their algorithmic DRAM bytes (signals, transform passes) */
-    uint64_t lag_reruns;           /* FP32 form: lag searches the f32 pass left undecided */
+    uint64_t lag_reruns;           /* lag searches that the f32 pass left undecided */
 } visqol_b200_timing;
 
 /* Score n pairs as visqol_measure_batch does; with traces non-NULL,
@@ -261,7 +261,7 @@ int visqol_b200_lag_search(const double *a, size_t la, const double *b, size_t l
 int visqol_b200_refine_lag(const double *s1, size_t l1, const double *s2, size_t l2, const float *approx,
                            size_t n, double scale, double tol, int64_t *lag, int32_t *decided);
 
-/* out[i] = num[i] / den[i] by the FP32 and FP64-FMA forms' NSIM quotient: a
+/* out[i] = num[i] / den[i] by the FAST and BALANCED forms' NSIM quotient: a
  * reciprocal estimate refined by Markstein's Newton-Raphson steps, then one
  * correction of the quotient. For den[i] > 0 in [2^-1000, 2^1000] the
  * result is within one ulp of the IEEE quotient. */
@@ -314,7 +314,7 @@ int visqol_b200_dp(const double *sims, size_t np, size_t nf_deg,
  * reference: it exists for callers that cannot allocate device memory at
  * call time (a process whose caching allocator already holds the free HBM,
  * or one that cannot let cudaFree wait for the whole device). Its device
- * buffers come from one ~6 MiB array reserved in the library image.
+ * buffers come from one ~5 MiB array reserved in the library image.
  * Limits: np <= 2048 and np * nf_deg <= 262144, else
  * VISQOL_E_INVALID_ARGUMENT. The first call on a device resolves the array
  * (make it before any stream capture); calls that overlap in time on one
