@@ -12,6 +12,8 @@ def test_one_copy_a_device(native, monkeypatch):
     """A context of its own kind first (tables, module loading, autotuning),
     then eight more of one lane each: beyond their arenas they take less than
     2 MB each, where a copy of the tables is over 4."""
+    import gc
+
     import torch
     from akvisqol_b200 import synth
     monkeypatch.setenv("VISQOL_GPU_LANES", "1")
@@ -23,6 +25,7 @@ def test_one_copy_a_device(native, monkeypatch):
         return ctx
 
     held = [context()]
+    gc.collect()  # no earlier context goes while the memory is counted
     free = torch.cuda.mem_get_info()[0]
     held += [context() for _ in range(8)]
     taken = free - torch.cuda.mem_get_info()[0]
